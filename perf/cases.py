@@ -304,7 +304,7 @@ def _prepare_layer(c, seed, dtype, gen):
                             slot_mapping=torch.tensor(slots, dtype=torch.int64, device=DEV), **meta)
     out = torch.empty((rows, c["heads"], 128), dtype=dtype, device=DEV)
     call.plan(q, out, kc, vc)
-    return dict(call=call, q=q, k=k, v=v, out=out, kc=kc, vc=vc)
+    return dict(call=call, q=q, k=k, v=v, out=out, kc=kc, vc=vc, ptab=ptab, ntab=ntab, stab=stab, slots=slots)
 
 
 class _Context:
@@ -336,7 +336,10 @@ def _prepare_iteration(c, seed, dtype, gen):
     q, k, v = _qkv(sum(fills) + len(suffix), c["heads"], 128, dtype, gen)
     model = [B200SharedPromptsGenerate(i, 128 ** -0.5, c["heads"], 128) for i in range(c["layers"])]
     config = types.SimpleNamespace(block_size=BLOCK, device="cuda:0", dtype=dtype)
-    return dict(jobs=jobs, kc=kc, vc=vc, caches=list(zip(kc, vc)), q=q, k=k, v=v, model=model, config=config)
+    slots = [x for n, t in zip(fills, tabs[1:]) for x in _slots(t, 0, n)]
+    slots += [_slots(t, n - 1, 1)[0] for n, t in zip(suffix, tabs[1 + len(fills):])]
+    return dict(jobs=jobs, kc=kc, vc=vc, caches=list(zip(kc, vc)), q=q, k=k, v=v, model=model, config=config, ptab=tabs[:1],
+                ntab=tabs[1:1 + len(fills)], stab=tabs[1 + len(fills):], slots=slots)
 
 
 def _prepare_paged(c, seed, dtype, gen):
@@ -357,7 +360,7 @@ def _prepare_shared(c, seed, dtype, gen):
     q, k, v = _qkv(len(suffix), c["heads"], 128, dtype, gen)
     slots = torch.tensor([_slots(t, n - 1, 1)[0] for n, t in zip(suffix, tabs[1:])], dtype=torch.int64, device=DEV)
     return dict(q=q, k=k, v=v, kc=kc, vc=vc, slots=slots, plen=plen, ptab=_i32([int(b) for b in tabs[0]]), ctx=_i32(suffix),
-                tables=_table(tabs[1:]))
+                tables=_table(tabs[1:]), stab=tabs[1:])
 
 
 def _prepare_host(c, seed, dtype, gen):
@@ -374,7 +377,7 @@ def _prepare_host(c, seed, dtype, gen):
     step.h_slots.copy_(torch.tensor([_slots(t, m - 1, 1)[0] for m, t in zip(suffix, tabs[1:])], dtype=torch.int64))
     step.h_suffix_tables.copy_(tables)
     step.h_suffix_lens.copy_(torch.tensor(suffix, dtype=torch.int32))
-    return dict(step=step, kc=kc, vc=vc)
+    return dict(step=step, kc=kc, vc=vc, ptab=tabs[:1], stab=tabs[1:])
 
 
 def _prepare_rotary(c, seed, dtype, gen):
@@ -450,3 +453,96 @@ def run(state):
         pb.move_tokens_from_blocked_v_cache(s.vc, s.v_rows, s.src, s.dst)
         return s.k_rows, s.v_rows
     return pb.sample_top_p(s.logits, s.temperature, s.top_p, uniforms=s.uniforms)
+
+
+# ---------------------------------------------------------------------------------------------
+# the same in 64 bits, by plain torch
+# ---------------------------------------------------------------------------------------------
+def _rows_of(kc, vc, blocks, n):
+    """Keys and values of a context's first n tokens, [n, heads, head_size] in 64 bits."""
+    ids = torch.as_tensor([int(b) for b in blocks[:_up(n)]], dtype=torch.int64, device=DEV)
+    k, v = kc[ids], vc[ids]
+    k = k.permute(0, 3, 1, 2, 4).reshape(len(ids) * BLOCK, kc.shape[1], -1)
+    v = v.permute(0, 3, 1, 2).reshape(len(ids) * BLOCK, vc.shape[1], -1)
+    return k[:n].double(), v[:n].double()
+
+
+def _fill(kc, vc, k, v, slots):
+    s = torch.as_tensor(slots, dtype=torch.int64, device=DEV)
+    rows = k.shape[0]
+    kc[s // BLOCK, :, :, s % BLOCK, :] = k.reshape(rows, kc.shape[1], kc.shape[2], kc.shape[4]).to(kc.dtype)
+    vc[s // BLOCK, :, :, s % BLOCK] = v.reshape(rows, vc.shape[1], vc.shape[2]).to(vc.dtype)
+
+
+def _attend(q, parts, out):
+    """Rows q [n, heads, d] over the keys and values of all parts; a part is (k, v, tokens each row sees or None)."""
+    scale = q.shape[2] ** -0.5
+    for lo in range(0, q.shape[1], 8):
+        h = slice(lo, lo + 8)
+        scores = []
+        for k, _, seen in parts:
+            x = torch.einsum("nhd,thd->hnt", q[:, h].double(), k[:, h]) * scale
+            if seen is not None:
+                x.masked_fill_(torch.arange(k.shape[0], device=DEV)[None, None, :] >= seen[None, :, None], float("-inf"))
+            scores.append(x)
+        p = torch.softmax(torch.cat(scores, dim=2), dim=2)
+        out[:, h] = torch.einsum("hnt,thd->nhd", p, torch.cat([v[:, h] for _, v, _ in parts]))
+
+
+def _exact_rows(q, kc, vc, prefix, ptab, group, suffix, stab, new, ntab):
+    """A batch: the prefills' rows first (under the first prefix, where there is one), then one row per sequence."""
+    out = torch.zeros(q.shape, dtype=torch.float64, device=DEV)
+    shared = [_rows_of(kc, vc, t, n) for t, n in zip(ptab, prefix)]
+    at = 0
+    for n, t in zip(new, ntab):
+        own = (*_rows_of(kc, vc, t, n), torch.arange(1, n + 1, device=DEV))
+        _attend(q[at:at + n], ([(*shared[0], None)] if shared else []) + [own], out[at:at + n])
+        at += n
+    for g, n, t in zip(group, suffix, stab):
+        _attend(q[at:at + 1], ([(*shared[g], None)] if g >= 0 else []) + [(*_rows_of(kc, vc, t, n), None)], out[at:at + 1])
+        at += 1
+    return out
+
+
+def exact(case, seed):
+    """What ``run`` returns, in 64 bits; None for moved bytes (the caches of an attention call) and token ids."""
+    c = case
+    if c["op"] in ("move", "sample"):
+        return None
+    s = prepare(case, seed)
+    if c["op"] == "rotary":
+        half = s.cos_sin.shape[1] // 2
+        cos, sin = (x[:, None, :].double() for x in s.cos_sin[s.positions].split(half, dim=1))
+
+        def turn(x):
+            a, b = x[..., :half].double(), x[..., half:].double()
+            return torch.cat([a * cos - b * sin, b * cos + a * sin], dim=-1)
+
+        kc = s.kc.double()
+        _fill(kc, s.vc, turn(s.k), s.v, s.slots)
+        return turn(s.q), kc, s.vc
+    if c["op"] == "paged":
+        share = c["heads"] // c["kv_heads"]
+        out = torch.zeros(s.q.shape, dtype=torch.float64, device=DEV)
+        for i, (n, t) in enumerate(zip(_lens(c), s.tables.tolist())):
+            k, v = (x.repeat_interleave(share, dim=1) for x in _rows_of(s.kc, s.vc, t, n))
+            _attend(s.q[i:i + 1], [(k, v, None)], out[i:i + 1])
+        return out
+    if c["op"] == "layer":
+        prefix, group, suffix, new = _layer_lens(c)
+        _fill(s.kc, s.vc, s.k, s.v, s.slots)
+        return _exact_rows(s.q, s.kc, s.vc, prefix, s.ptab, group, suffix, s.stab, new, s.ntab), None, None
+    plen, suffix, fills = _lens(c)
+    group = [0] * len(suffix)
+    if c["op"] == "iteration":
+        outs = []
+        for kc, vc in s.caches:
+            _fill(kc, vc, s.k, s.v, s.slots)
+            outs.append(_exact_rows(s.q, kc, vc, [plen], s.ptab, group, suffix, s.stab, fills, s.ntab).flatten(1))
+        return outs, None, None
+    if c["op"] == "shared":
+        _fill(s.kc, s.vc, s.k, s.v, s.slots)
+        return _exact_rows(s.q, s.kc, s.vc, [plen], [s.ptab.tolist()], group, suffix, s.stab, [], []), None, None
+    h = s.step
+    _fill(s.kc, s.vc, h.h_key_new.to(DEV), h.h_value_new.to(DEV), h.h_slots.to(DEV))
+    return _exact_rows(h.h_query.to(DEV), s.kc, s.vc, [plen], s.ptab, group, suffix, s.stab, [], []), None, None
