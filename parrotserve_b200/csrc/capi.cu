@@ -186,6 +186,12 @@ int validate_and_bind(const pb_attn_params* p, WsLayout* L, AttnDev* d) {
   d->acc = reinterpret_cast<float*>(ws + L->off_acc);
   d->scale_log2e = p->scale * kLog2e;
   d->num_rows = p->num_rows; d->num_heads = p->num_heads; d->num_kv_heads = p->num_kv_heads;
+  // Grouped kv heads: the largest divisor of heads / kv heads up to 8 (the columns of the MMA), so that all
+  // items of a kv head hold equally many query heads. Only a call with a head mapping shares kv heads.
+  d->gqa_heads = 1;
+  if (p->head_mapping && p->num_heads % p->num_kv_heads == 0)
+    for (int n = 2; n <= 8; ++n)
+      if ((p->num_heads / p->num_kv_heads) % n == 0) d->gqa_heads = n;
   d->num_groups = p->num_groups;
   d->suffix_table_stride = p->suffix_table_stride; d->group_table_stride = p->group_table_stride;
   d->parts = L->parts; d->pparts = L->pparts; d->sparts = L->sparts; d->cs = L->cs; d->cp = L->cp;

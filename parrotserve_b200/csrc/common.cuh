@@ -300,6 +300,7 @@ struct AttnDev {            // what the attention kernels read
   const void* value_new;
   int64_t key_new_stride, value_new_stride;
   int32_t slot_is_i64;
+  int32_t gqa_heads;          // query heads of one kv head that the 16-bit single-query kernel takes in one item (1: no sharing)
   int32_t out_vec16;          // 1: output rows may be written with 16-byte stores (base and row stride aligned)
   int64_t q_stride, out_stride, kv_block_stride, kv_head_stride, num_blocks;
 };

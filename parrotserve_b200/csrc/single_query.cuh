@@ -21,6 +21,8 @@
 namespace pb {
 namespace {
 
+constexpr int kMaxItemHeads = 8;  // query heads of one kv head that the GQA form takes at once: the N of mma.m16n8k16
+
 template <typename T, int D, int B>
 struct SqCfg {
   static constexpr int kVec = ElemTraits<T>::kVec;          // elements per 16 bytes
@@ -43,6 +45,12 @@ struct SqCfg {
   static_assert(kStageBytes % 128 == 0, "stage alignment");
   static_assert(kKChunks >= 1 && kAcc >= 1, "shape");
   static constexpr int warp_bytes(int ns) { return ns * kStageBytes + 128 /*p*/ + ns * 16 /*meta*/ + 64 /*bars*/ ; }
+  // GQA form of the MMA consumer: stages hold the two tiles alone; the query rows of an item (up to
+  // kMaxItemHeads) go to one of two slots of their own, because three stages with eight rows each do not
+  // fit eight warps into shared memory
+  static constexpr int kGqaStageBytes = 2 * kTileBytes;
+  static constexpr int kQSlotBytes = kMaxItemHeads * kQBytes;
+  static constexpr int gqa_warp_bytes(int ns) { return ns * kGqaStageBytes + 2 * kQSlotBytes + ns * 16 /*meta*/ + 64 /*bars*/; }
 };
 
 struct ItemState {
@@ -117,17 +125,28 @@ __device__ __forceinline__ void ldmatrix_x4(uint32_t* r, uint32_t addr) {
 //   the B operand of  O = V.p  needs, so P never moves between lanes. p enters as an exact
 //   (hi + lo) pair of 16-bit values. This cuts the instruction stream per 8 KiB of KV about 5x,
 //   which is what kept the FMA consumer from saturating HBM.
-template <typename T, int D, int B, int WARPS, int NS, bool MMA>
+//
+// GQA (MMA consumer only): an item is (row, chunk, d.gqa_heads query heads of ONE kv head). Their rows
+//   are rows 0..7 of the A operand of S = q.K^T, and the lanes' logits are again the B operand of
+//   O = V.p, whose eight columns are the heads: the same instructions that served one head serve up to
+//   eight, and every K/V tile is read once for all of them instead of once per query head. What bounds
+//   it is HBM. 128 sequences of 16..2048 tokens, 32 query over 8 kv heads (536 MB): 307 us with one head
+//   per item, 116 us so (4.6 TB/s of the bytes, one-shot call with its planner included).
+template <typename T, int D, int B, int WARPS, int NS, bool MMA, bool GQA>
 __global__ void __launch_bounds__((WARPS + 1) * 32, 1) sq_attn_kernel(const AttnDev d) {
+  static_assert(MMA || !GQA, "only the MMA consumer takes several heads at once");
   using C = SqCfg<T, D, B>;
   extern __shared__ __align__(128) uint8_t smem_raw[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  constexpr int kWarpBytes = (C::warp_bytes(NS) + 127) / 128 * 128;
+  constexpr int kWarpBytes = ((GQA ? C::gqa_warp_bytes(NS) : C::warp_bytes(NS)) + 127) / 128 * 128;
+  constexpr int kStage = GQA ? C::kGqaStageBytes : C::kStageBytes;
+  constexpr int kOffMeta = GQA ? NS * kStage + 2 * C::kQSlotBytes : NS * kStage + 128;  // behind the q slots / the p buffer
   WorkQueue* wq = reinterpret_cast<WorkQueue*>(smem_raw + WARPS * kWarpBytes);
   uint8_t* wbase = smem_raw + (warp < WARPS ? warp : 0) * kWarpBytes;
-  float* pbuf = reinterpret_cast<float*>(wbase + NS * C::kStageBytes);
-  int4* meta = reinterpret_cast<int4*>(wbase + NS * C::kStageBytes + 128);
-  uint64_t* bars = reinterpret_cast<uint64_t*>(wbase + NS * C::kStageBytes + 128 + NS * 16);
+  float* pbuf = reinterpret_cast<float*>(wbase + NS * kStage);  // (FMA consumer)
+  uint8_t* qslots = wbase + NS * kStage;                        // (GQA)
+  int4* meta = reinterpret_cast<int4*>(wbase + kOffMeta);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(wbase + kOffMeta + NS * 16);
 
   if (lane == 0 && warp < WARPS) {
 #pragma unroll
@@ -145,7 +164,16 @@ __global__ void __launch_bounds__((WARPS + 1) * 32, 1) sq_attn_kernel(const Attn
   // and only waits for it at the very end, so the merge sees both complete.
   if (d.sq_waits_at_start) pdl_wait();
   pdl_trigger();
-  const int H = d.num_heads;
+  // Query heads per item. The head mapping lives in device memory: several heads share an item only if
+  // it is the usual one (head h reads kv head h / (heads / kv heads)); otherwise items hold one head.
+  int hpi = 1;
+  if constexpr (GQA) {
+    const int share = d.num_heads / d.num_kv_heads;
+    bool usual = true;
+    for (int h = threadIdx.x; h < d.num_heads; h += (WARPS + 1) * 32) usual = usual && d.head_mapping[h] == h / share;
+    if (__syncthreads_and(usual)) hpi = d.gqa_heads;
+  }
+  const int H = d.num_heads / hpi;  // items per list entry
   const long long n_items = (long long)d.hdr[kHdrNumSq] * H;
   // Asked to perform the KV fill, but the lists were built without the new-token slots: no item
   // carries a token, the fill would silently not happen. Recorded as a fault (NaN output).
@@ -186,7 +214,7 @@ __global__ void __launch_bounds__((WARPS + 1) * 32, 1) sq_attn_kernel(const Attn
       if (lane < cnt) {
         const long long id = base + lane;
         const int sc = (int)(id / H);
-        head = (int)(id - (long long)sc * H);
+        head = (int)(id - (long long)sc * H) * hpi;
         a = *reinterpret_cast<const int4*>(&d.sq_items[sc]);        // row, meta, ntok, part
         b = *(reinterpret_cast<const int4*>(&d.sq_items[sc]) + 1);  // bid[4]
       }
@@ -275,7 +303,7 @@ __global__ void __launch_bounds__((WARPS + 1) * 32, 1) sq_attn_kernel(const Attn
     const long long id0 = (long long)blockIdx.x * WARPS + warp;
     if (id0 < n_items) {
       const int sc = (int)(id0 / H);
-      const int head = (int)(id0 - (long long)sc * H);
+      const int head = (int)(id0 - (long long)sc * H) * hpi;
       const int4 a = *reinterpret_cast<const int4*>(&d.sq_items[sc]);        // row, meta, ntok, part
       const int4 b = *(reinterpret_cast<const int4*>(&d.sq_items[sc]) + 1);  // bid[4]
       cur.row = a.x; cur.head = head; cur.kvh = d.head_mapping ? d.head_mapping[head] : head;
@@ -294,6 +322,7 @@ __global__ void __launch_bounds__((WARPS + 1) * 32, 1) sq_attn_kernel(const Attn
   }
   int p_blk = 0;
   uint32_t issued = 0, consumed = 0;
+  uint32_t q_issued = 0, q_consumed = 0;                // (GQA) items whose query rows were asked for / taken
 
   const size_t esz = sizeof(T);
   const uint64_t kv_policy = l2_policy_evict_first();
@@ -325,6 +354,7 @@ __global__ void __launch_bounds__((WARPS + 1) * 32, 1) sq_attn_kernel(const Attn
   while (true) {
     // ------------------------------ producer ------------------------------
     while (issued - consumed < (uint32_t)NS && cur.nblk > 0) {
+      if (GQA && p_blk == 0 && q_issued - q_consumed == 2) break;  // both q slots wait for their items to start
       const int s = issued % NS;
       if (p_blk > 0 && (p_blk & 31) == 0)  // chunks longer than 32 blocks: next window of ids
         cur_bid = (p_blk + lane < cur.nblk) ? cur.tbl[p_blk + lane] : 0;
@@ -338,17 +368,17 @@ __global__ void __launch_bounds__((WARPS + 1) * 32, 1) sq_attn_kernel(const Attn
         const bool nw = last && cur.has_new && d.key_new != nullptr;  // this block ends with the row's new token
         const int ntok_blk = min(B, cur.ntok - p_blk * B);
         meta[s] = make_int4(cur.row, cur.head | (cur.part << 16), blk,
-                            ntok_blk | (first ? 256 : 0) | (last ? 512 : 0) | (nw ? 1024 : 0));
+                            ntok_blk | (first ? 256 : 0) | (last ? 512 : 0) | (nw ? 1024 : 0) | (GQA && (q_issued & 1) ? 2048 : 0));
         const uint32_t bar = smem_u32(&bars[s]);
-        const uint32_t dst = smem_u32(wbase + s * C::kStageBytes);
+        const uint32_t dst = smem_u32(wbase + s * kStage);
         const size_t off = ((size_t)blk * d.kv_block_stride + (size_t)cur.kvh * d.kv_head_stride) * esz;
-        mbar_arrive_expect_tx(bar, 2 * C::kTileBytes + (first ? C::kQBytes : 0) + (nw ? 2 * C::kQBytes : 0));
+        mbar_arrive_expect_tx(bar, 2 * C::kTileBytes + (first ? (GQA ? hpi : 1) * C::kQBytes : 0) + (nw ? 2 * C::kQBytes : 0));
         // the K and V tiles are read once per call: first out of L2, so that the partials and tables stay
         bulk_g2s_hint(dst, kc + off, C::kTileBytes, bar, kv_policy);
         bulk_g2s_hint(dst + C::kTileBytes, vc + off, C::kTileBytes, bar, kv_policy);
         if (first)
-          bulk_g2s(dst + 2 * C::kTileBytes,
-                   qg + ((size_t)cur.row * d.q_stride + (size_t)cur.head * D) * esz, C::kQBytes, bar);
+          bulk_g2s(GQA ? smem_u32(qslots + (q_issued & 1) * C::kQSlotBytes) : dst + 2 * C::kTileBytes,
+                   qg + ((size_t)cur.row * d.q_stride + (size_t)cur.head * D) * esz, (GQA ? hpi : 1) * C::kQBytes, bar);
         if (nw) {  // the new key and value rows of (row, head) ride along with the block they belong in
           bulk_g2s(dst + 2 * C::kTileBytes + C::kQBytes,
                    reinterpret_cast<const uint8_t*>(d.key_new) + ((size_t)cur.row * d.key_new_stride + (size_t)cur.head * D) * esz,
@@ -359,6 +389,7 @@ __global__ void __launch_bounds__((WARPS + 1) * 32, 1) sq_attn_kernel(const Attn
         }
       }
       ++issued;
+      if (GQA && p_blk == 0) ++q_issued;
       ++p_blk;
       if (p_blk == cur.nblk) {
         cur = pop(cur_bid);
@@ -378,9 +409,9 @@ __global__ void __launch_bounds__((WARPS + 1) * 32, 1) sq_attn_kernel(const Attn
     const int4 mt = meta[s];
     const int ntok_blk = mt.w & 255;
     const int it_row = mt.x, it_head = mt.y & 0xffff, it_part = mt.y >> 16;
-    const uint8_t* stage = wbase + s * C::kStageBytes;
+    const uint8_t* stage = wbase + s * kStage;
 
-    if (mt.w & 1024) {
+    if (!GQA && (mt.w & 1024)) {
       // KV fill of the row's new token, fused: its key and value rows arrived with the block. They
       // replace the (not yet written) last token of this copy of the block and go into the cache
       // itself, where later calls find them (with identity head mapping this warp is the only one
@@ -406,7 +437,98 @@ __global__ void __launch_bounds__((WARPS + 1) * 32, 1) sq_attn_kernel(const Attn
       __syncwarp();
     }
 
-    if constexpr (MMA) {
+    if constexpr (GQA) {
+      // The consumer below with several heads: lane (g, t) = (lane / 4, lane % 4) holds row g (head g of the
+      // item) of S and columns 2t, 2t + 1 (heads 2t, 2t + 1) of O. Rows and columns beyond the item's
+      // heads carry zeros that are never stored.
+      const uint32_t st_addr = smem_u32(stage);
+      const int g = lane >> 2;
+      if (mt.w & 256) {
+        const uint32_t* qs = reinterpret_cast<const uint32_t*>(qslots + ((mt.w & 2048) ? C::kQSlotBytes : 0)) + g * (D / 2);
+#pragma unroll
+        for (int kk = 0; kk < kKSteps; ++kk) {
+          qa[kk][0] = g < hpi ? qs[kk * 8 + quad_t] : 0u;
+          qa[kk][1] = g < hpi ? qs[kk * 8 + 4 + quad_t] : 0u;
+        }
+        ++q_consumed;
+        m_run = m_true = -INFINITY;
+        l_run = 0.f;
+#pragma unroll
+        for (int j = 0; j < kKSteps; ++j) oacc[j][0] = oacc[j][1] = oacc[j][2] = oacc[j][3] = 0.f;
+      }
+      float sa[4] = {0.f, 0.f, 0.f, 0.f}, sb[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int kk = 0; kk < kKSteps; ++kk) {
+        uint32_t kb[4];
+        ldmatrix_x4(kb, st_addr + ldm_k_off + kk * 512);
+        const uint32_t a[4] = {qa[kk][0], 0u, qa[kk][1], 0u};
+        MmaOps<T>::mma(sa, a, kb[0], kb[1]);
+        MmaOps<T>::mma(sb, a, kb[2], kb[3]);
+      }
+      float lg[4] = {sa[0] * d.scale_log2e, sa[1] * d.scale_log2e, sb[0] * d.scale_log2e, sb[1] * d.scale_log2e};
+      if (ntok_blk < B) {
+        if (2 * quad_t >= ntok_blk) lg[0] = -INFINITY;
+        if (2 * quad_t + 1 >= ntok_blk) lg[1] = -INFINITY;
+        if (8 + 2 * quad_t >= ntok_blk) lg[2] = -INFINITY;
+        if (9 + 2 * quad_t >= ntok_blk) lg[3] = -INFINITY;
+      }
+      float bm = fmaxf(fmaxf(lg[0], lg[1]), fmaxf(lg[2], lg[3]));
+      bm = fmaxf(bm, __shfl_xor_sync(0xffffffffu, bm, 1));
+      bm = fmaxf(bm, __shfl_xor_sync(0xffffffffu, bm, 2));  // the maximum of head g over the block
+      m_true = fmaxf(m_true, bm);
+      const bool grow = bm > m_run + 8.f;  // lazy reference maximum, per head
+      if (__any_sync(0xffffffffu, grow)) {
+        const float alpha = grow ? fast_exp2(m_run - bm) : 1.f;
+        l_run *= alpha;
+        if (grow) m_run = bm;
+        const float a0 = __shfl_sync(0xffffffffu, alpha, 8 * quad_t), a1 = __shfl_sync(0xffffffffu, alpha, 8 * quad_t + 4);
+#pragma unroll
+        for (int j = 0; j < kKSteps; ++j) { oacc[j][0] *= a0; oacc[j][1] *= a1; oacc[j][2] *= a0; oacc[j][3] *= a1; }
+      }
+      float p[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) p[i] = fast_exp2(lg[i] - m_run);
+      l_run += (p[0] + p[1]) + (p[2] + p[3]);
+      uint32_t hi0, lo0, hi1, lo1;
+      MmaOps<T>::split(p[0], p[1], hi0, lo0);
+      MmaOps<T>::split(p[2], p[3], hi1, lo1);
+      if (ntok_blk < B) {  // ragged last block: 0 * (stale bytes) has to stay 0
+        uint16_t* vz = reinterpret_cast<uint16_t*>(const_cast<uint8_t*>(stage) + C::kTileBytes);
+        for (int dd = lane; dd < D; dd += 32)
+          for (int tk = ntok_blk; tk < B; ++tk) vz[dd * B + tk] = 0;
+        fence_proxy_async_smem();
+        __syncwarp();
+      }
+#pragma unroll
+      for (int j = 0; j < kKSteps; ++j) {
+        uint32_t va[4];
+        ldmatrix_x4(va, st_addr + C::kTileBytes + ldm_v_off + j * 512);
+        MmaOps<T>::mma(oacc[j], va, hi0, hi1);
+        MmaOps<T>::mma(oacc[j], va, lo0, lo1);
+      }
+      __syncwarp();  // stage s and the q slot may be overwritten from here on
+      if (mt.w & 512) {
+        const float fix = fast_exp2(m_run - m_true);
+        float l = l_run * fix;
+        l += __shfl_xor_sync(0xffffffffu, l, 1);
+        l += __shfl_xor_sync(0xffffffffu, l, 2);
+        const float f0 = __shfl_sync(0xffffffffu, fix, 8 * quad_t), f1 = __shfl_sync(0xffffffffu, fix, 8 * quad_t + 4);
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          const int hh = 2 * quad_t + c;
+          if (hh < hpi) {
+            float* ap = d.acc + partial_slot(d, it_row, it_part, it_head + hh) * D + g;
+            const float f = c ? f1 : f0;
+#pragma unroll
+            for (int j = 0; j < kKSteps; ++j) {
+              ap[16 * j] = oacc[j][c] * f;
+              ap[16 * j + 8] = oacc[j][2 + c] * f;
+            }
+          }
+        }
+        if (quad_t == 0 && g < hpi) d.ml[partial_slot(d, it_row, it_part, it_head + g)] = make_float2(m_true, l);
+      }
+    } else if constexpr (MMA) {
       const uint32_t st_addr = smem_u32(stage);
       if (mt.w & 256) {  // first block of an item: fresh accumulators, q as row 0 of the A fragments
         const uint32_t* qs = reinterpret_cast<const uint32_t*>(stage + 2 * C::kTileBytes);
@@ -606,13 +728,15 @@ __global__ void __launch_bounds__((WARPS + 1) * 32, 1) sq_attn_kernel(const Attn
   if (!d.sq_waits_at_start) pdl_wait();  // the dense prefix kernel has completed
 }
 
-template <typename T, int D, int B, int WARPS, int NS, bool MMA>
+template <typename T, int D, int B, int WARPS, int NS, bool MMA, bool GQA = false>
 cudaError_t launch_sq(const AttnDev& d, cudaStream_t s) {
   using C = SqCfg<T, D, B>;
-  constexpr int kWarpBytes = (C::warp_bytes(NS) + 127) / 128 * 128;
+  if constexpr (MMA && !GQA)
+    if (d.gqa_heads > 1) return launch_sq<T, D, B, WARPS, NS, true, true>(d, s);
+  constexpr int kWarpBytes = ((GQA ? C::gqa_warp_bytes(NS) : C::warp_bytes(NS)) + 127) / 128 * 128;
   constexpr int smem = WARPS * kWarpBytes + (int)sizeof(WorkQueue);
   static_assert(smem <= 227 * 1024, "shared memory budget");
-  auto kfn = sq_attn_kernel<T, D, B, WARPS, NS, MMA>;
+  auto kfn = sq_attn_kernel<T, D, B, WARPS, NS, MMA, GQA>;
   cudaError_t e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
   return launch_kernel(kfn, d.num_sms, (WARPS + 1) * 32, smem, s, true, d);

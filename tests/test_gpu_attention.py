@@ -178,6 +178,29 @@ def test_head_mapping_gqa():
     assert_close_to_oracle(out, ref, torch.float16, "gqa")
 
 
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("kv,share,d", [(2, 2, 128), (1, 3, 128), (2, 4, 80), (1, 5, 64), (3, 8, 128), (1, 12, 96), (2, 16, 256), (1, 7, 112)])
+@pytest.mark.parametrize("usual", [True, False])
+def test_several_query_heads_per_item(dtype, kv, share, d, usual):
+    """Query heads that share a kv head are taken together (2..8 at once), under the usual mapping; under any
+    other one each is an item of its own. Contexts of one block (the query slots of a warp run full), of one
+    token, of whole and ragged blocks, of several chunks, and empty; strided query rows."""
+    sl = [1] * 24 + [15, 16, 17, 0, 64, 65, 200, 1000] + [9] * 40
+    _, kc, vc, meta = _mini(dtype, kv, 0, sl, nb=256, seed=60, groups=[], d=d)
+    g = torch.Generator(device=DEV).manual_seed(61)
+    heads = kv * share
+    q = torch.randn((len(sl), 2 * heads * d), generator=g, device=DEV).to(dtype)[:, :heads * d].view(len(sl), heads, d)
+    hm = [h // share for h in range(heads)]
+    if not usual:
+        hm = [(h * 5 + 1) % kv for h in range(heads)]
+        hm[0], hm[-1] = kv - 1, 0
+    i32 = lambda a: torch.tensor(a, dtype=torch.int32, device=DEV)
+    out = pb.vllm_paged_attention(q, kc, vc, i32(hm), i32(sl), i32(meta["st"]))
+    ref = orc.gold_grouped_attention(q.float().cpu(), kc.float().cpu(), vc.float().cpu(), None, None, None, sl, meta["st"],
+                                     head_mapping=hm)
+    assert_close_to_oracle(out, ref, dtype, f"{share} query heads per kv head, head size {d}")
+
+
 def test_prev_post_native_entry_points():
     """prev writes normalised out + base-2 stats; post merges a second context into it in place:
     prev(A) then post(B) == attention over A ++ B (csrc/attention.cpp:19-47)."""
