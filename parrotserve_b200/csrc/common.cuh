@@ -75,8 +75,7 @@ struct DnItem {       // one tile of query rows and the kv tokens they attend in
   // request's own context (seg_tables + tbl2_off, nblk/ntok/causal_base above). nt1 == 0: one piece,
   // in group_tables (causal_base == 0) or seg_tables (causal_base > 0) at tbl_off.
   int32_t nt1, nblk1, ntok1, tbl2_off;
-  int32_t flags;  // kDnDirect: none of the item's rows has any other partial (no suffix, no item of
-                  // its own), so a CTA that holds ALL kv tiles of (item, head) writes the finished,
+  int32_t flags;  // kDnDirect: none of the item's rows has any other partial (no suffix, no other item), so a CTA that holds ALL kv tiles of (item, head) writes the finished,
                   // normalised output rows itself and the merge skips them
   int32_t pad[3];
 };

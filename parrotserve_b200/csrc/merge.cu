@@ -16,39 +16,83 @@ namespace {
 constexpr int kMergeWarps = 4;
 constexpr int kPairLanes = 16;                 // lanes that share one (row, head)
 constexpr int kPairsPerWarp = 32 / kPairLanes;  // two (row, head) pairs per warp: twice the loads in flight
+constexpr int kPairs = kMergeWarps * kPairsPerWarp;  // heads a CTA works on at once
+constexpr int kMaxHeadsPerCta = kMergeWarps * 32;    // one thread each finds a head's partials
+constexpr int kManyRows = 1024;                      // from here on one CTA takes up to kMaxHeadsPerCta heads of a row
 
-template <typename T, int D>
-__global__ void __launch_bounds__(kMergeWarps * 32) merge_kernel(const AttnDev d) {
+// dense_cta_of_tile, with a 32-bit division wherever the product fits: the 64-bit one is a routine of some
+// hundred instructions, and every (row, head) asks twice.
+__device__ __forceinline__ int cta_of_tile(long long g, long long total, int ctas) {
+  const int c = dense_active_ctas(total, ctas);
+  if (total < (1ll << 24)) return (int)(((uint32_t)(g + 1) * (uint32_t)c + (uint32_t)(total - 1)) / (uint32_t)total) - 1;
+  return dense_cta_of_tile(g, total, ctas);
+}
+static_assert((1ull << 24) * (kMaxSMs + 1) < (1ull << 32), "the 32-bit product must fit");
+
+// kMany == false: a CTA per eight heads of a row; the lanes of a (row, head) find its partials for themselves.
+// kMany == true (prefill): a CTA per row (and 128 heads) walks its heads eight at a time. How many
+// partials a head has is worked out by one thread per head; a row that the dense kernel has finished leaves at
+// once. (With a CTA per eight pairs, all lanes dividing, a batch of ten thousand prefill rows spent 100 us on
+// finding out that there was nothing to do. For few rows the detour through shared memory costs 1.5 us.)
+template <typename T, int D, bool kMany>
+__global__ void __launch_bounds__(kMergeWarps * 32) merge_kernel(const AttnDev d, const int heads_per_cta) {
+  // (kMany) partials of each head: prefix, segment, outer prefix; w: 1 = finished by the dense kernel
+  extern __shared__ int4 parts_of[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int sub = lane % kPairLanes;  // position inside the pair's lane group
-  const long long idx = ((long long)blockIdx.x * kMergeWarps + warp) * kPairsPerWarp + lane / kPairLanes;
   const int H = d.num_heads;
+  const int per_row = (H + heads_per_cta - 1) / heads_per_cta;  // CTAs of a row, next to each other
+  const int row = blockIdx.x / per_row, h_lo = (blockIdx.x - row * per_row) * heads_per_cta, h_hi = min(H, h_lo + heads_per_cta);
   // The planner's output (row_info, dense items, header) is older than the attention kernels of
   // this call, so it is read while they still run; only then wait for their partials.
-  const bool active = idx < (long long)d.num_rows * H;
-  const int row = active ? (int)(idx / H) : 0, head = active ? (int)(idx - (long long)row * H) : 0;
   const RowInfo info = d.row_info[row];
-  // partials of the row: [prefix][causal segment][suffix]; a dense stage leaves one partial per
-  // CTA that touched the (row tile, head), the single-query kernel one per chunk
   const long long total = d.hdr[kHdrDnTiles];
   const int dctas = dense_ctas_of(d);
-  auto dense_parts = [&](int dn) {
-    const DnItem it = d.dn_items[dn];
-    const long long g0 = (long long)it.tile_base + (long long)head * it.nt;
-    return dense_cta_of_tile(g0 + it.nt - 1, total, dctas) - dense_cta_of_tile(g0, total, dctas) + 1;
+  // partials of the row: [prefix][causal segment][suffix]; a dense stage leaves one partial per
+  // CTA that touched the (row tile, head), the single-query kernel one per chunk
+  auto parts = [&](int head) {
+    auto dense_parts = [&](int dn) {
+      const int nt = d.dn_items[dn].nt;
+      const long long g0 = (long long)d.dn_items[dn].tile_base + (long long)head * nt;
+      return cta_of_tile(g0 + nt - 1, total, dctas) - cta_of_tile(g0, total, dctas) + 1;
+    };
+    int4 p;
+    p.x = (info.dn >= 0) ? dense_parts(info.dn) : info.np_sq;
+    p.y = (info.seg_dn >= 0) ? dense_parts(info.seg_dn) : info.nc_sq;
+    p.z = (info.odn >= 0) ? dense_parts(info.odn) : info.onp_sq;  // outer-prefix partials
+    // rows the dense kernel finished by itself (their only partial, held whole by one CTA): nothing to do
+    const int only = (info.dn >= 0 && p.x == 1 && p.y == 0) ? info.dn : (info.seg_dn >= 0 && p.y == 1 && p.x == 0) ? info.seg_dn : -1;
+    p.w = (only >= 0 && info.nsc == 0 && p.z == 0 && dense_direct_ok(d, d.dn_items[only])) ? 1 : 0;
+    return p;
   };
-  const int np = (info.dn >= 0) ? dense_parts(info.dn) : info.np_sq;
-  const int nc = (info.seg_dn >= 0) ? dense_parts(info.seg_dn) : info.nc_sq;
-  // rows the dense kernel finished by itself (its only partial, held whole by one CTA): nothing to do
-  const int no = (info.odn >= 0) ? dense_parts(info.odn) : info.onp_sq;  // outer-prefix partials
-  const bool direct = active && info.dn >= 0 && np == 1 && nc == 0 && info.nsc == 0 && no == 0 &&
-                      dense_direct_ok(d, d.dn_items[info.dn]);
+  int4 mine = make_int4(0, 0, 0, 0);
+  bool any_open = true;
+  if (kMany) {
+    bool open = false;
+    if ((int)threadIdx.x < h_hi - h_lo) {
+      mine = parts(h_lo + threadIdx.x);
+      parts_of[threadIdx.x] = mine;
+      open = mine.w == 0;
+    }
+    any_open = __syncthreads_or(open);
+  } else {
+    const int head = h_lo + warp * kPairsPerWarp + lane / kPairLanes;
+    if (head < h_hi) mine = parts(head);
+  }
   pdl_wait();  // every partial of the prefix and suffix stages is complete and visible
   if (blockIdx.x == 0 && threadIdx.x == 0) d.hdr[kHdrSqCounter] = 0;  // ready for the next layer call
   // A call whose kernels recorded a fault (a wait that ran out, an index outside the cache, a list
   // that did not fit) has results that cannot be trusted: every output row becomes NaN, so that the
   // fault cannot pass unnoticed into the sampler even if nobody reads the status word.
   const bool poison = __ldcg(&d.hdr[kHdrStatus]) != kStatusOk;
+  if (kMany && !any_open && !poison) return;
+  for (int hb = h_lo; hb < (kMany ? h_hi : h_lo + 1); hb += kPairs) {
+  const int head = hb + warp * kPairsPerWarp + lane / kPairLanes;
+  const bool active = head < h_hi;
+  if (kMany) mine = active ? parts_of[head - h_lo] : make_int4(0, 0, 0, 0);
+  const int np = mine.x, nc = mine.y, no = mine.z;
+  const bool direct = mine.w != 0;
+  const long long idx = (long long)row * H + head;
   const int n = (active && !direct) ? np + nc + info.nsc + no : 0;
   int n_warp = n;  // the two pairs of a warp walk their partials in lockstep
 #pragma unroll
@@ -83,7 +127,7 @@ __global__ void __launch_bounds__(kMergeWarps * 32) merge_kernel(const AttnDev d
   // were addressed with it), so the next kernel in the stream may become resident: an attention
   // kernel or a KV fill waits for this grid's completion before it touches anything, and a planner
   // only overwrites the lists read above and completes after this grid.
-  pdl_trigger();
+  if (hb == h_lo) pdl_trigger();
 
   float4 o4[kPer];
 #pragma unroll
@@ -129,7 +173,7 @@ __global__ void __launch_bounds__(kMergeWarps * 32) merge_kernel(const AttnDev d
   }
 #pragma unroll
   for (int o = kPairLanes / 2; o >= 1; o >>= 1) L += __shfl_xor_sync(0xffffffffu, L, o);
-  if (!active || (direct && !poison)) return;
+  if (!active || (direct && !poison)) continue;
   if (l_prev > 0.f) {
     const float w = fast_exp2(m_prev - M) * l_prev;
     L += w;
@@ -161,21 +205,28 @@ __global__ void __launch_bounds__(kMergeWarps * 32) merge_kernel(const AttnDev d
     d.qk_max[idx] = M;
     d.exp_sum[idx] = L;
   }
+  }  // heads
+}
+
+template <typename T, int D>
+cudaError_t launch_merge_d(const AttnDev& d, cudaStream_t s) {
+  const bool many = d.num_rows >= kManyRows;
+  const int hpc = !many ? kPairs : d.num_heads < kMaxHeadsPerCta ? d.num_heads : kMaxHeadsPerCta;
+  const unsigned grid = (unsigned)((long long)d.num_rows * ((d.num_heads + hpc - 1) / hpc));
+  return many ? launch_kernel(merge_kernel<T, D, true>, grid, kMergeWarps * 32, (size_t)hpc * sizeof(int4), s, true, d, hpc)
+              : launch_kernel(merge_kernel<T, D, false>, grid, kMergeWarps * 32, 0, s, true, d, hpc);
 }
 
 template <typename T>
 cudaError_t launch_merge_t(const AttnDev& d, int head_size, cudaStream_t s) {
-  const long long n = (long long)d.num_rows * d.num_heads;
-  if (n == 0) return cudaSuccess;
-  const long long per_cta = (long long)kMergeWarps * kPairsPerWarp;
-  const unsigned grid = (unsigned)((n + per_cta - 1) / per_cta);
+  if (d.num_rows == 0) return cudaSuccess;
   switch (head_size) {
-    case 64: return launch_kernel(merge_kernel<T, 64>, grid, kMergeWarps * 32, 0, s, true, d);
-    case 80: return launch_kernel(merge_kernel<T, 80>, grid, kMergeWarps * 32, 0, s, true, d);
-    case 96: return launch_kernel(merge_kernel<T, 96>, grid, kMergeWarps * 32, 0, s, true, d);
-    case 112: return launch_kernel(merge_kernel<T, 112>, grid, kMergeWarps * 32, 0, s, true, d);
-    case 128: return launch_kernel(merge_kernel<T, 128>, grid, kMergeWarps * 32, 0, s, true, d);
-    case 256: return launch_kernel(merge_kernel<T, 256>, grid, kMergeWarps * 32, 0, s, true, d);
+    case 64: return launch_merge_d<T, 64>(d, s);
+    case 80: return launch_merge_d<T, 80>(d, s);
+    case 96: return launch_merge_d<T, 96>(d, s);
+    case 112: return launch_merge_d<T, 112>(d, s);
+    case 128: return launch_merge_d<T, 128>(d, s);
+    case 256: return launch_merge_d<T, 256>(d, s);
     default: return cudaErrorInvalidValue;
   }
 }

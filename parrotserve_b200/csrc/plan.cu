@@ -370,7 +370,8 @@ __global__ void __launch_bounds__(kPlanThreads, 1) plan_kernel(const AttnDev d, 
         const int vis = seg_tile_visible(d, p, rt);
         DnItem it;
         it.nt1 = it.nblk1 = it.ntok1 = it.tbl2_off = 0;
-        it.flags = 0; it.pad[0] = it.pad[1] = it.pad[2] = 0;
+        it.flags = kDnDirect;  // withdrawn below if a row of the tile has a prefix or a suffix besides
+        it.pad[0] = it.pad[1] = it.pad[2] = 0;
         it.row0 = p.r0 + rt * RT;
         it.nrows = min(RT, p.n - rt * RT);
         it.tbl_off = s * d.seg_table_stride;
@@ -466,8 +467,12 @@ __global__ void __launch_bounds__(kPlanThreads, 1) plan_kernel(const AttnDev d, 
       }
     }
     d.row_info[r] = info;
-    if ((nsc > 0 || info.odn >= 0 || info.onp_sq > 0) && info.dn >= 0 && (d.dn_items[info.dn].flags & kDnDirect))
-      atomicAnd(&d.dn_items[info.dn].flags, ~kDnDirect);  // this row needs the merge: so does its tile
+    // this row has other partials and needs the merge: so does its tile
+    const bool other = nsc > 0 || info.odn >= 0 || info.onp_sq > 0;
+    if (info.dn >= 0 && (other || info.seg_dn >= 0) && (d.dn_items[info.dn].flags & kDnDirect))
+      atomicAnd(&d.dn_items[info.dn].flags, ~kDnDirect);
+    if (info.seg_dn >= 0 && (other || info.dn >= 0 || info.np_sq > 0) && (d.dn_items[info.seg_dn].flags & kDnDirect))
+      atomicAnd(&d.dn_items[info.seg_dn].flags, ~kDnDirect);
     // The row's new token (a pure decode batch whose fill the suffix kernel performs itself): it must be
     // the last token of the row's suffix, so that the item of the last chunk can carry it.
     bool carries_new = false;

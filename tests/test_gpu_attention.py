@@ -320,6 +320,48 @@ def test_causal_segments_with_cached_context(dtype, d, row_tile):
 
 
 @pytest.mark.parametrize("row_tile", [128, 256])
+@pytest.mark.parametrize("extra,plen", [(0, 0), (400, 0), (400, 40)])
+def test_prefills_without_a_dense_prefix_finish_in_the_dense_kernel(row_tile, extra, plen):
+    """Row tiles of a prefill whose rows have no other partial are finished by the dense kernel; tiles of at
+    most 64 rows, split tiles and tiles with one row that also has a suffix or a prefix read by the
+    single-query kernel still go through the merge. `extra` more decode rows take the batch over the row
+    count from which the merge walks up to 128 heads of a row per CTA."""
+    b, h, d, dtype = 16, 9, 128, torch.float16
+    segs = [(0, 65), (33, 128), (0, 200), (7, 64), (0, 300)]  # (cached tokens, new tokens)
+    seg_offs = np.cumsum([0] + [n for _, n in segs]).tolist()
+    seg_kv = [c + n for c, n in segs]
+    rows = seg_offs[-1] + 20 + extra
+    slens = [0] * seg_offs[-1] + [1 + i % 40 for i in range(20 + extra)]
+    slens[seg_offs[2] + 130] = 21  # one row of the third request's second tile
+    need = sum((n + b - 1) // b for n in seg_kv + slens) + 8
+    perm = np.random.default_rng(70).permutation(need).tolist()
+    blocks = lambda n: [perm.pop() for _ in range((n + b - 1) // b)]
+    g = torch.Generator(device=DEV).manual_seed(71)
+    kc = torch.randn((need, h, d // 8, b, 8), generator=g, device=DEV).to(dtype)
+    vc = torch.randn((need, h, d, b), generator=g, device=DEV).to(dtype)
+    q = torch.randn((rows, h, d), generator=g, device=DEV).to(dtype)
+    seg_tabs, stabs, ptab = [blocks(n) for n in seg_kv], [blocks(n) for n in slens], blocks(plen)
+    pad = lambda rr: [r + [0] * (max(len(x) for x in rr) - len(r)) for r in rr]
+    i32 = lambda a: torch.tensor(a, dtype=torch.int32, device=DEV)
+    kw, okw = {}, [None, None, None]
+    if plen:  # two rows of the fifth request: a group too small for the tensor cores
+        okw = [[seg_offs[4], seg_offs[4] + 2], [plen], [ptab]]
+        kw = dict(group_row_offsets=i32(okw[0]), group_prefix_lens=i32(okw[1]), group_tables=i32(okw[2]))
+    call = pb.AttentionCall(num_rows=rows, num_heads=h, head_size=d, block_size=b, dtype=dtype, device=q.device,
+                            suffix_lens=i32(slens), suffix_tables=i32(pad(stabs)), seg_row_offsets=i32(seg_offs),
+                            seg_kv_lens=i32(seg_kv), seg_tables=i32(pad(seg_tabs)), dense_row_tile=row_tile, **kw)
+    out = torch.full_like(q, float("nan"))
+    call.run(q, out, kc, vc)
+    assert call.status() == 0
+    some = sorted({r for o in seg_offs[:-1] for r in (o, o + 1, o + 63)} | {seg_offs[2] + 129, seg_offs[2] + 130, seg_offs[5] - 1, rows - 1}
+                  | set(range(0, rows, 29)))
+    ref = orc.gold_grouped_attention(q.float().cpu(), kc.float().cpu(), vc.float().cpu(), *okw, slens, pad(stabs), rows=some,
+                                     seg_row_offsets=seg_offs, seg_kv_lens=seg_kv, seg_tables=pad(seg_tabs))
+    assert torch.isfinite(out).all()
+    assert_close_to_oracle(out[some], ref, dtype, f"prefills alone, {rows} rows")
+
+
+@pytest.mark.parametrize("row_tile", [128, 256])
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 def test_causal_segments_joined_straddling_and_outside_groups(dtype, row_tile):
     """The planner's cases around prefill requests and prefix groups: requests inside a dense group
