@@ -202,10 +202,13 @@ int validate_and_bind(const pb_attn_params* p, WsLayout* L, AttnDev* d) {
   // Read by the planner only: the split is part of the plan.
   d->num_sms = sm_count();
   d->dense_ctas = p->dense_ctas > 0 ? (p->dense_ctas < d->num_sms ? p->dense_ctas : d->num_sms) : 0;
-  // Rows per dense item. Row-tile pairs pay when most of the dense work comes in tiles of 128 rows
-  // (prefill, large groups); a decode batch with small groups keeps single row tiles, where the
-  // rows of a tile are duplicated so that several threads share a row's exponentials.
-  d->dense_row_tile = p->dense_row_tile > 0 ? p->dense_row_tile : 128;
+  // Rows per dense item. Row-tile pairs pay in batches of prefill requests of more than 128 rows each (32 x 140
+  // rows, 32 heads: 180 us against 197 with single tiles; 4 x 2192: 439 against 485; under a 512-token
+  // prefix 32 x 140: 295 against 338). Requests of at most 128 rows leave half of the pair kernel's softmax
+  // threads idle (32 x 128 under that prefix: 238 against 199), and with few rows in all the single tiles
+  // spread over more SMs (1 x 256: 37 against 35; 1 x 1000: 71 against 76).
+  d->dense_row_tile = p->dense_row_tile > 0 ? p->dense_row_tile
+                      : (p->num_segments > 0 && p->num_rows >= 1000 && (long long)p->num_rows > 128ll * p->num_segments) ? 256 : 128;
   d->q_stride = p->q_stride; d->out_stride = p->out_stride;
   d->out_vec16 = (aligned16(p->out) && (p->out_stride * elem_bytes(p->dtype)) % 16 == 0) ? 1 : 0;
   d->acc_tma = 0;

@@ -17,7 +17,7 @@ constexpr float kLog2e = 1.4426950408889634f;
 // Workspace layout. Everything a call needs beyond its inputs and outputs lives here.
 //
 //   header   int32[64]   [0] status word, [1] number of single-query work items,
-//                        [2] number of dense (tensor-core) work items, [3] dense kv tiles * heads,
+//                        [2] number of dense (tensor-core) work items, [3] length of the dense tile order,
 //                        [4] next unclaimed single-query work item (reset by the planner and the merge),
 //                        [5] CTAs of the dense kernel that take work (the planner's split of the SMs, or
 //                        the caller's dense_ctas as it was when the lists were built),
@@ -33,9 +33,11 @@ constexpr float kLog2e = 1.4426950408889634f;
 // prefix partial c uses j = c, partial c of the
 // row's causal segment uses j = pparts + c, suffix chunk c uses j = pparts + cparts + c.
 //
-// Dense tile order ("stream-K"): item i, head h, kv tile t has index tile_base_i + h * nt_i + t;
-// CTA c of the dense kernel owns [c * total / ctas, (c + 1) * total / ctas). A (item, head) that
-// several CTAs touch gets one partial per CTA, numbered in CTA order (dense_first_cta below).
+// Dense tile order ("stream-K"): item i, head h, kv tile t has index tile_base_i + h * (fixed_i + nt_i) +
+// fixed_i + t; CTA c of the dense kernel owns [c * total / ctas, (c + 1) * total / ctas). A (item, head)
+// that several CTAs touch gets one partial per CTA, numbered in CTA order (dense_cta_of_tile below). The
+// fixed_i positions before the tiles of a causal item hold no tile: they stand for what an (item, head)
+// costs beside its tiles (kCausalFixedTiles below).
 // ---------------------------------------------------------------------------------------------
 struct SqItem {       // one (row, kv chunk); the kernel multiplies the list by the heads
   int32_t row;
@@ -67,7 +69,7 @@ struct DnItem {       // one tile of query rows and the kv tokens they attend in
   int32_t nblk;       // blocks of the last piece
   int32_t ntok;       // tokens of the last piece
   int32_t nt;         // 128-token kv tiles of the whole item (both pieces)
-  int32_t tile_base;  // index of (this item, head 0, kv tile 0) in the global dense tile order
+  int32_t tile_base;  // first index of (this item, head 0) in the global dense tile order
   int32_t causal_base;  // 0: every row sees all tokens of the last piece;
                         // > 0: row i of the tile sees its first causal_base + i tokens (causal segment)
   // Two-piece items (a prefill request inside a prefix group): kv tiles [0, nt1) walk the group's
@@ -77,10 +79,18 @@ struct DnItem {       // one tile of query rows and the kv tokens they attend in
   int32_t nt1, nblk1, ntok1, tbl2_off;
   int32_t flags;  // kDnDirect: none of the item's rows has any other partial (no suffix, no other item), so a CTA that holds ALL kv tiles of (item, head) writes the finished,
                   // normalised output rows itself and the merge skips them
-  int32_t pad[3];
+  int32_t fixed;  // positions of the tile order in front of every head's tiles (kCausalFixedTiles or 0)
+  int32_t pad[2];
 };
 static_assert(sizeof(DnItem) == 64, "DnItem must be 64 bytes");
 constexpr int32_t kDnDirect = 1;
+// What one (item, head) costs beside its kv tiles, in tiles: the load of Q, the first tile's way through the
+// pipeline, the epilogue. Causal items have from one kv tile to dozens, so CTAs with equal shares of the
+// tiles alone had very unequal work (those with the short row tiles of a prefill up to ten times as many
+// epilogues, and the SMs were busy 54 % of the kernel's time). Four prompts of 1500..3000 tokens: 645 us with
+// 0, 483 with 2, 485 with 3, 488 with 5; 16 prefills under a shared prefix are indifferent to 2 (1226).
+// Items without a causal mask are equally long within a group; their tiles are split as they are.
+constexpr int32_t kCausalFixedTiles = 2;
 constexpr int32_t kDnOuter = 2;   // the item walks an outer prefix group (outer_tables, outer partial range)
 
 struct WsLayout {

@@ -228,18 +228,23 @@ struct SegmentWalker {
     next_base = (i + 1 < n_dn) ? (long long)d.dn_items[i + 1].tile_base : total;
   }
   __device__ bool next(Segment& sg) {
-    if (g >= g_end) return false;
-    while (g >= next_base && idx + 1 < n_dn) load(idx + 1);
-    sg.it = cur;
-    const long long rel = g - sg.it.tile_base;
-    sg.head = (int)(rel / sg.it.nt);
-    sg.t0 = (int)(rel - (long long)sg.head * sg.it.nt);
-    const long long room = g_end - g;
-    sg.t1 = (int)min((long long)sg.it.nt, sg.t0 + room);
-    const long long g0 = (long long)sg.it.tile_base + (long long)sg.head * sg.it.nt;
-    sg.part = dense_cta_of_tile(g, total, ctas) - dense_cta_of_tile(g0, total, ctas);
-    g += sg.t1 - sg.t0;
-    return true;
+    while (g < g_end) {
+      while (g >= next_base && idx + 1 < n_dn) load(idx + 1);
+      const int len = cur.fixed + cur.nt;  // positions of one head
+      const long long rel = g - cur.tile_base;
+      sg.head = (int)(rel / len);
+      const int u0 = (int)(rel - (long long)sg.head * len);
+      const int u1 = (int)min((long long)len, u0 + (g_end - g));
+      g += u1 - u0;
+      if (u1 <= cur.fixed) continue;  // this CTA's share ends before the head's first tile
+      sg.it = cur;
+      sg.t0 = max(u0 - cur.fixed, 0);
+      sg.t1 = u1 - cur.fixed;
+      const long long g0 = (long long)cur.tile_base + (long long)sg.head * len + cur.fixed;  // the head's first tile
+      sg.part = dense_cta_of_tile(g0 + sg.t0, total, ctas) - dense_cta_of_tile(g0, total, ctas);
+      return true;
+    }
+    return false;
   }
 };
 

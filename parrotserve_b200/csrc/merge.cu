@@ -52,8 +52,8 @@ __global__ void __launch_bounds__(kMergeWarps * 32) merge_kernel(const AttnDev d
   // CTA that touched the (row tile, head), the single-query kernel one per chunk
   auto parts = [&](int head) {
     auto dense_parts = [&](int dn) {
-      const int nt = d.dn_items[dn].nt;
-      const long long g0 = (long long)d.dn_items[dn].tile_base + (long long)head * nt;
+      const int nt = d.dn_items[dn].nt, fixed = d.dn_items[dn].fixed;
+      const long long g0 = (long long)d.dn_items[dn].tile_base + (long long)head * (fixed + nt) + fixed;
       return cta_of_tile(g0 + nt - 1, total, dctas) - cta_of_tile(g0, total, dctas) + 1;
     };
     int4 p;

@@ -218,7 +218,7 @@ __global__ void __launch_bounds__(kPlanThreads, 1) plan_kernel(const AttnDev d, 
                       },
                       [&](int, const SegPlan& sp) {
                         my_dng += sp.n_rt;
-                        for (int rt = 0; rt < sp.n_rt; ++rt) my_tiles_g += p.nt + seg_tiles(d, sp, rt, B);
+                        for (int rt = 0; rt < sp.n_rt; ++rt) my_tiles_g += kCausalFixedTiles + p.nt + seg_tiles(d, sp, rt, B);
                       });
     } else {
       my_sq += p.npc * p.n_rows;
@@ -233,7 +233,7 @@ __global__ void __launch_bounds__(kPlanThreads, 1) plan_kernel(const AttnDev d, 
     if (seg_joined_group(d, p, B, dense_ok) >= 0) continue;  // counted with its group
     if (dense_ok) {
       my_dns += p.n_rt;
-      for (int rt = 0; rt < p.n_rt; ++rt) my_tiles_s += seg_tiles(d, p, rt, B);
+      for (int rt = 0; rt < p.n_rt; ++rt) my_tiles_s += kCausalFixedTiles + seg_tiles(d, p, rt, B);
     } else {
       for (int i = 0; i < p.n; ++i) {
         const int nb = (p.kv - p.n + i + 1 + B - 1) / B;
@@ -323,7 +323,7 @@ __global__ void __launch_bounds__(kPlanThreads, 1) plan_kernel(const AttnDev d, 
               it.tile_base = tile_g_base * d.num_heads;
               it.causal_base = 0;
               it.nt1 = it.nblk1 = it.ntok1 = it.tbl2_off = 0;
-              it.flags = 0; it.pad[0] = it.pad[1] = it.pad[2] = 0;
+              it.flags = 0; it.fixed = it.pad[0] = it.pad[1] = 0;
               tile_g_base += it.nt;
               d.dn_items[dng_base++] = it;
             }
@@ -340,13 +340,13 @@ __global__ void __launch_bounds__(kPlanThreads, 1) plan_kernel(const AttnDev d, 
               it.ntok1 = p.plen;
               it.tbl2_off = sidx * d.seg_table_stride;
               it.flags = kDnDirect;  // withdrawn below if a row of the tile turns out to have a suffix
-              it.pad[0] = it.pad[1] = it.pad[2] = 0;
+              it.fixed = kCausalFixedTiles; it.pad[0] = it.pad[1] = 0;
               it.nblk = (vis + B - 1) / B;
               it.ntok = vis;
               it.nt = p.nt + seg_tiles(d, sp, rt, B);
               it.tile_base = tile_g_base * d.num_heads;
               it.causal_base = sp.kv - sp.n + rt * RT + 1;  // own tokens row 0 of the tile sees
-              tile_g_base += it.nt;
+              tile_g_base += it.fixed + it.nt;
               d.dn_items[dng_base++] = it;
             }
           });
@@ -371,7 +371,7 @@ __global__ void __launch_bounds__(kPlanThreads, 1) plan_kernel(const AttnDev d, 
         DnItem it;
         it.nt1 = it.nblk1 = it.ntok1 = it.tbl2_off = 0;
         it.flags = kDnDirect;  // withdrawn below if a row of the tile has a prefix or a suffix besides
-        it.pad[0] = it.pad[1] = it.pad[2] = 0;
+        it.fixed = kCausalFixedTiles; it.pad[0] = it.pad[1] = 0;
         it.row0 = p.r0 + rt * RT;
         it.nrows = min(RT, p.n - rt * RT);
         it.tbl_off = s * d.seg_table_stride;
@@ -380,7 +380,7 @@ __global__ void __launch_bounds__(kPlanThreads, 1) plan_kernel(const AttnDev d, 
         it.nt = (it.nblk + kDenseTileBlocks - 1) / kDenseTileBlocks;
         it.tile_base = tile_s_base * d.num_heads;
         it.causal_base = p.kv - p.n + rt * RT + 1;  // tokens row 0 of the tile sees
-        tile_s_base += it.nt;
+        tile_s_base += it.fixed + it.nt;
         d.dn_items[dns_base++] = it;
       }
     } else {
@@ -411,7 +411,7 @@ __global__ void __launch_bounds__(kPlanThreads, 1) plan_kernel(const AttnDev d, 
         it.tile_base = tile_o_base * d.num_heads;
         it.causal_base = 0;
         it.nt1 = it.nblk1 = it.ntok1 = it.tbl2_off = 0;
-        it.flags = kDnOuter; it.pad[0] = it.pad[1] = it.pad[2] = 0;
+        it.flags = kDnOuter; it.fixed = it.pad[0] = it.pad[1] = 0;
         tile_o_base += it.nt;
         d.dn_items[dno_base++] = it;
       }
