@@ -172,6 +172,14 @@ __device__ __forceinline__ bool wait_or_abort(uint32_t bar, uint32_t parity, vol
   return __all_sync(0xffffffffu, ok);
 }
 
+// Two fp32 multiply-adds in one instruction, each rounded like fmaf.
+__device__ __forceinline__ void fma_pair(float& x, float& y, float scale, float add) {
+  asm("{\n\t.reg .b64 a, s, c;\n\t"
+      "mov.b64 a, {%0, %1};\n\tmov.b64 s, {%2, %2};\n\tmov.b64 c, {%3, %3};\n\t"
+      "fma.rn.f32x2 a, a, s, c;\n\tmov.b64 {%0, %1}, a;\n\t}"
+      : "+f"(x), "+f"(y) : "f"(scale), "f"(add));
+}
+
 template <typename T> struct Pack;
 template <> struct Pack<__half> {
   static __device__ __forceinline__ uint32_t two(float a, float b) {

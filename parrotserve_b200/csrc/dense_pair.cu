@@ -96,8 +96,10 @@ template <typename T, bool kMasked>
 __device__ __forceinline__ void exp_pack32(const uint32_t* v, int nvalid, float scale, float m, float* sum, uint32_t* out) {
 #pragma unroll
   for (int i = 0; i < 32; i += 2) {
-    float e0 = fast_exp2(fmaf(__uint_as_float(v[i]), scale, -m));
-    float e1 = fast_exp2(fmaf(__uint_as_float(v[i + 1]), scale, -m));
+    float e0 = __uint_as_float(v[i]), e1 = __uint_as_float(v[i + 1]);
+    fma_pair(e0, e1, scale, -m);  // (a packed instruction: four prompts of 1500..3000 tokens 440 -> 432 us)
+    e0 = fast_exp2(e0);
+    e1 = fast_exp2(e1);
     if (kMasked) {
       e0 = (i < nvalid) ? e0 : 0.f;
       e1 = (i + 1 < nvalid) ? e1 : 0.f;
