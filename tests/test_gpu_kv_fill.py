@@ -111,6 +111,28 @@ def test_fill_prefill_sized_batch_bit_exact(dtype, b):
     assert not bits(k2)[~keep].any()
 
 
+# Windows of 16 tokens with none, one, two and more runs starting in them; runs at even and odd offsets, of one
+# token, of a whole block, across windows; a token outside the cache; the last window cut short.
+RUNS = [[(0, 16)], [(16, 16), (37, 11), (32, 3)], [(49, 15), (64, 16), (81, 7)], [(95, 1), (97, 1), (99, 1), (101, 2), (120, 8)],
+        [(131, 29), (160, 32), (193, 14), (-1, 1), (208, 1)], [(9999, 1), (225, 5), (-1, 1), (-1, 1), (230, 10), (255, 1), (240, 3)]]
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+@pytest.mark.parametrize("h,d", [(1, 128), (5, 64), (4, 80), (3, 256)])
+@pytest.mark.parametrize("case", range(len(RUNS) + 1))
+def test_fill_windows(dtype, h, d, case):
+    b, nb = 16, 16
+    kc, vc, g = _caches(dtype, nb, h, d, b, 20)
+    runs = RUNS[case] if case < len(RUNS) else sum(RUNS, [])
+    slots = np.asarray([s + (i if s >= 0 else 0) for s, n in runs for i in range(n)], dtype=np.int64)
+    qkv = torch.randn((len(slots), 3, h, d), generator=g, device=DEV).to(dtype)
+    _, key, value = qkv.unbind(dim=1)
+    kr, vr = bits(kc).copy(), bits(vc).copy()
+    orc.fill_reference(bits(key), bits(value), kr, vr, np.where(slots < nb * b, slots, -1))
+    pb.vllm_reshape_and_cache(key, value, kc, vc, torch.tensor(slots, device=DEV))
+    assert np.array_equal(bits(kc), kr) and np.array_equal(bits(vc), vr)
+
+
 def test_fill_config4_shape_and_decode_reference_layout():
     wl = make_workload(4, shrink=8, num_heads=4)
     t = wl.materialize(DEV)
@@ -150,6 +172,30 @@ def test_move_tokens_from_blocked_caches(dtype):
     assert np.array_equal(bits(kd), ke) and np.array_equal(bits(vd), ve)
     with pytest.raises(AssertionError):
         pb.move_tokens_from_blocked_k_cache(kc, kd, torch.tensor(src, device=DEV), torch.tensor(dst[:-1], device=DEV))
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+@pytest.mark.parametrize("h,d", [(1, 128), (5, 64), (9, 80), (3, 256)])
+@pytest.mark.parametrize("n", [1, 15, 16, 17, 150])
+def test_move_runs_from_blocked_caches(dtype, h, d, n):
+    """Runs of consecutive slots (whole blocks, odd offsets, across the 16 entries a CTA looks at), lone slots in
+    any order, and entries outside the cache or the destination, which are left out."""
+    nb, b = 16, 16
+    kc, vc, g = _caches(dtype, nb, h, d, b, 30)
+    slots = [s + (i if 0 <= s < nb * b else 0) for s, m in sum(RUNS, []) for i in range(m)]
+    src = np.asarray((slots[40:] + slots[:40])[:n] if n > 1 else [77])
+    rows = 200
+    dst = np.random.default_rng(31).permutation(rows)[:n]
+    if n > 16:
+        dst[3], dst[12] = -1, rows  # outside the destination
+    kd, vd = (torch.randn((rows, h, d), generator=g, device=DEV).to(dtype) for _ in range(2))
+    ke, ve = bits(kd).copy(), bits(vd).copy()
+    ok = (src >= 0) & (src < nb * b) & (dst >= 0) & (dst < rows)
+    kg, vg = orc.gather_reference(bits(kc), bits(vc), src[ok])
+    ke[dst[ok]], ve[dst[ok]] = kg, vg
+    pb.move_tokens_from_blocked_k_cache(kc, kd, torch.tensor(src, device=DEV), torch.tensor(dst, device=DEV))
+    pb.move_tokens_from_blocked_v_cache(vc, vd, torch.tensor(src, device=DEV), torch.tensor(dst, device=DEV))
+    assert np.array_equal(bits(kd), ke) and np.array_equal(bits(vd), ve)
 
 
 @pytest.mark.parametrize("dtype,h,d", [(torch.float16, 96, 128), (torch.float32, 3, 20), (torch.bfloat16, 1, 7)])
