@@ -29,6 +29,20 @@ template <int E> struct ElemOf;
 template <> struct ElemOf<2> { using type = uint16_t; };
 template <> struct ElemOf<4> { using type = uint32_t; };
 
+// Runs of a list of slots: lane l of the warp holds entry first - 1 + l (its slot, or a negative number
+// outside the list). A run is a maximal stretch of entries with consecutive slots inside one block of 16;
+// bit l of `cont` says that entry l continues the run of the entry before it. A run that starts in lanes
+// 1..16 ends in lane 31 at the latest.
+__device__ __forceinline__ unsigned run_continues(long long slot) {
+  const long long before = __shfl_up_sync(0xffffffffu, slot, 1);
+  const bool cont = (threadIdx.x & 31) > 0 && slot > 0 && before >= 0 && slot == before + 1 && (slot & 15) != 0;
+  return __ballot_sync(0xffffffffu, cont);
+}
+__device__ __forceinline__ int run_length(unsigned cont, int lane_of_first) {
+  const unsigned rest = lane_of_first < 31 ? cont >> (lane_of_first + 1) : 0u;
+  return __ffs(~rest);  // 1 + trailing ones (bit 31 of `rest` is never set)
+}
+
 // FILL == true : scatter rows into the cache.   FILL == false : gather rows out of the cache.
 template <int E, bool FILL>
 __global__ void __launch_bounds__(kFillWarps * 32) kv_run_kernel(
@@ -317,18 +331,209 @@ __global__ void __launch_bounds__(kFillWarps * 32) rotary_fill_kernel(
   }
 }
 
-// Runs of a list of slots: lane l of the warp holds entry first - 1 + l (its slot, or a negative number
-// outside the list). A run is a maximal stretch of entries with consecutive slots inside one block of 16;
-// bit l of `cont` says that entry l continues the run of the entry before it. A run that starts in lanes
-// 1..16 ends in lane 31 at the latest.
-__device__ __forceinline__ unsigned run_continues(long long slot) {
-  const long long before = __shfl_up_sync(0xffffffffu, slot, 1);
-  const bool cont = (threadIdx.x & 31) > 0 && slot > 0 && before >= 0 && slot == before + 1 && (slot & 15) != 0;
-  return __ballot_sync(0xffffffffu, cont);
-}
-__device__ __forceinline__ int run_length(unsigned cont, int lane_of_first) {
-  const unsigned rest = lane_of_first < 31 ? cont >> (lane_of_first + 1) : 0u;
-  return __ffs(~rest);  // 1 + trailing ones (bit 31 of `rest` is never set)
+// KV fill at block size 16, with (ROT) or without NeoX rotation of q and k: a CTA takes 16 consecutive
+// tokens and kWinHeads heads; every thread owns one (token, chunk) and walks the heads, so that the loads of
+// all of them are in flight together and the cos/sin values are read once for them. q and k need no more
+// than the token's own slot: neighbouring lanes are neighbouring tokens, whose cells of a block are
+// neighbours too. V goes from rows to tiles [d][16 tokens]: two tokens of a run share a 4-byte word, so a
+// thread reads the same chunk of both, and eight lanes write one whole 32-byte row of the tile; nothing goes
+// through shared memory. The runs that START among the CTA's tokens are written by it up to their end, so
+// that a full block's sectors are written whole; a window with more than kFewRuns of them (decode tokens) is
+// written token by token. What bounds it is memory. 10 842 tokens (16
+// prefills, 240 decodes) x 32 heads, fp16: rotary and fill 165 -> 118 us (4.5 TB/s of 534 MB) against a CTA per
+// token of which fifteen of sixteen left at once; the plain fill of 8767 prefill tokens about 65 -> 52 us.
+// Heads per CTA: rotary 2: 125 us, 4: 118; plain fill 4: 430 us with the attention behind it, 2: 426. At most 96
+// registers (five CTAs an SM): 129 us; q in CTAs of its own: 130 us.
+constexpr int kFewRuns = 2;
+
+constexpr int win_heads(bool rot) { return rot ? 4 : 2; }
+
+template <typename T, bool ROT>
+__global__ void __launch_bounds__(128) fill_window_kernel(
+    uint8_t* __restrict__ query, uint8_t* __restrict__ key, const uint8_t* __restrict__ value,
+    uint8_t* __restrict__ kcache, uint8_t* __restrict__ vcache, const void* __restrict__ slots, const int is64,
+    const long long* __restrict__ positions, const uint8_t* __restrict__ cos_sin, const int rot_dim,
+    const long long max_pos, const long long T_tok, const int Hq, const int H, const int D,
+    const long long q_stride, const long long key_stride, const long long value_stride, const long long kbs,
+    const long long khs, const long long num_blocks, const int write_key_back) {
+  constexpr int B = 16;
+  constexpr int kWinHeads = win_heads(ROT);
+  constexpr int E = (int)sizeof(T);
+  constexpr int kVec = 16 / E;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const long long first = (long long)blockIdx.x * 16;
+  const int h0 = blockIdx.y * kWinHeads;
+  // resident while the kernel before this one drains: wait for it before reading anything, then let the
+  // next kernel set itself up (it waits before it reads the cache)
+  pdl_wait();
+  pdl_trigger();
+  const int nch = D / kVec;                       // 16-byte chunks per (token, head) row
+  const int half = ROT ? rot_dim / kVec / 2 : 0;  // chunks in each half of the rotated part
+  auto cs_row = [&](long long tok) {
+    long long pos = positions[tok];
+    pos = pos < 0 ? 0 : (pos >= max_pos ? max_pos - 1 : pos);  // clamped: never read outside the table
+    return cos_sin + (size_t)pos * rot_dim * E;
+  };
+  // rotates the chunk pair u of one token's rows of this CTA's heads: dst_x / dst_y(head) say where to
+  auto rotate_rows = [&](const uint8_t* row0, int heads, const uint8_t* cs, int u, auto&& store) {
+    uint4 x[kWinHeads], y[kWinHeads];
+#pragma unroll
+    for (int k = 0; k < kWinHeads; ++k) {
+      if (h0 + k < heads) {
+        const uint4* row = reinterpret_cast<const uint4*>(row0 + (size_t)(h0 + k) * D * E);
+        x[k] = row[u];
+        y[k] = row[u + half];
+      }
+    }
+    float fc[kVec], fs[kVec];
+    unpack16<T>(__ldg(reinterpret_cast<const uint4*>(cs) + u), fc);
+    unpack16<T>(__ldg(reinterpret_cast<const uint4*>(cs) + half + u), fs);
+#pragma unroll
+    for (int k = 0; k < kWinHeads; ++k) {
+      if (h0 + k < heads) {
+        float fx[kVec], fy[kVec], rx[kVec], ry[kVec];
+        unpack16<T>(x[k], fx);
+        unpack16<T>(y[k], fy);
+#pragma unroll
+        for (int j = 0; j < kVec; ++j) {
+          rx[j] = fx[j] * fc[j] - fy[j] * fs[j];
+          ry[j] = fy[j] * fc[j] + fx[j] * fs[j];
+        }
+        store(h0 + k, pack16<T>(rx), pack16<T>(ry));
+      }
+    }
+  };
+
+  if (ROT) {  // q in place; with no cache k too (eight lanes: 128 contiguous bytes of a row)
+    const long long tok = first + warp * 4 + (lane >> 3);
+    if (tok < T_tok) {
+      const uint8_t* cs = cs_row(tok);
+      for (int u = lane & 7; u < half; u += 8) {
+        uint8_t* qrow = query + (size_t)tok * q_stride * E;
+        rotate_rows(qrow, Hq, cs, u, [&](int h, const uint4& ox, const uint4& oy) {
+          uint4* row = reinterpret_cast<uint4*>(qrow + (size_t)h * D * E);
+          row[u] = ox;
+          row[u + half] = oy;
+        });
+        if (kcache == nullptr) {
+          uint8_t* krow = key + (size_t)tok * key_stride * E;
+          rotate_rows(krow, H, cs, u, [&](int h, const uint4& ox, const uint4& oy) {
+            uint4* row = reinterpret_cast<uint4*>(krow + (size_t)h * D * E);
+            row[u] = ox;
+            row[u + half] = oy;
+          });
+        }
+      }
+    }
+    if (kcache == nullptr) return;
+  }
+  if (h0 >= H) return;
+
+  // lane l: the slot of token first - 1 + l (negative: none, or outside the cache)
+  const long long my = first - 1 + lane;
+  long long slot = (my >= 0 && my < T_tok) ? load_slot(slots, is64, my) : -1;
+  if (slot >= num_blocks * B) slot = -1;
+
+  // ---- K: token `i` of the window, chunks g, g + 8, ... ----
+  const int i = (lane & 7) + 8 * (warp & 1), g = (lane >> 3) + 4 * (warp >> 1);
+  const long long s_i = __shfl_sync(0xffffffffu, slot, i + 1);
+  if (s_i >= 0) {
+    uint8_t* krow = key + (size_t)(first + i) * key_stride * E;
+    uint4* cell0 = reinterpret_cast<uint4*>(kcache + (size_t)(s_i / B) * kbs * E) + (s_i & (B - 1));
+    auto cell = [&](int h) { return reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(cell0) + (size_t)h * khs * E); };
+    if (ROT) {
+      const uint8_t* cs = cs_row(first + i);
+      for (int u = g; u < half; u += 8)
+        rotate_rows(krow, H, cs, u, [&](int h, const uint4& ox, const uint4& oy) {
+          cell(h)[(size_t)u * B] = ox;
+          cell(h)[(size_t)(u + half) * B] = oy;
+          if (write_key_back) {
+            uint4* row = reinterpret_cast<uint4*>(krow + (size_t)h * D * E);
+            row[u] = ox;
+            row[u + half] = oy;
+          }
+        });
+    }
+#pragma unroll 2
+    for (int c = 2 * half + g; c < nch; c += 8) {
+      uint4 v[kWinHeads];
+#pragma unroll
+      for (int k = 0; k < kWinHeads; ++k)
+        if (h0 + k < H) v[k] = reinterpret_cast<const uint4*>(krow + (size_t)(h0 + k) * D * E)[c];
+#pragma unroll
+      for (int k = 0; k < kWinHeads; ++k)
+        if (h0 + k < H) cell(h0 + k)[(size_t)c * B] = v[k];
+    }
+  }
+
+  // ---- V: the runs that start among tokens first .. first + 15 (lanes 1 .. 16) ----
+  const unsigned cont = run_continues(slot);
+  const unsigned starts = ~cont & __ballot_sync(0xffffffffu, slot >= 0) & 0x1fffeu;
+  if (starts == 0) return;
+  if (E == 2 && __popc(starts) <= kFewRuns) {
+    for (unsigned left = starts; left; left &= left - 1) {
+      const int at = __ffs(left) - 1, run = run_length(cont, at);
+      const long long s0 = __shfl_sync(0xffffffffu, slot, at);
+      const int off = (int)(s0 & (B - 1));
+      const int pair = lane & 7;  // positions 2 pair, 2 pair + 1 of the block
+      const int ia = 2 * pair - off, ib = ia + 1;
+      const bool in_a = ia >= 0 && ia < run, in_b = ib >= 0 && ib < run;
+      if (!in_a && !in_b) continue;
+      const uint8_t* rows = value + (size_t)(first - 1 + at + (in_a ? ia : ib)) * value_stride * E;
+      const size_t next = (in_a && in_b) ? (size_t)value_stride * E : 0;
+      uint8_t* tile = vcache + ((size_t)(s0 / B) * kbs + (size_t)h0 * khs) * E + pair * 4;
+      for (int c = (lane >> 3) + 4 * warp; c < nch; c += 16) {
+        uint4 a[kWinHeads], b[kWinHeads];
+#pragma unroll
+        for (int k = 0; k < kWinHeads; ++k) {
+          if (h0 + k < H) {
+            const uint8_t* p = rows + (size_t)(h0 + k) * D * E + c * 16;
+            a[k] = __ldg(reinterpret_cast<const uint4*>(p));
+            b[k] = __ldg(reinterpret_cast<const uint4*>(p + next));
+          }
+        }
+#pragma unroll
+        for (int k = 0; k < kWinHeads; ++k) {
+          if (h0 + k < H) {
+            uint8_t* out = tile + (size_t)k * khs * E + c * kVec * 32;
+            const uint32_t av[4] = {a[k].x, a[k].y, a[k].z, a[k].w}, bv[4] = {b[k].x, b[k].y, b[k].z, b[k].w};
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+              const uint32_t w = __byte_perm(av[j >> 1], bv[j >> 1], (j & 1) ? 0x7632 : 0x5410);
+              if (in_a && in_b) *reinterpret_cast<uint32_t*>(out + j * 32) = w;
+              else *reinterpret_cast<uint16_t*>(out + j * 32 + (in_a ? 0 : 2)) = (uint16_t)(in_a ? w : w >> 16);
+            }
+          }
+        }
+      }
+    }
+    return;
+  }
+  // token by token: lanes [lo, hi) are the tokens of those runs
+  const int last = 31 - __clz(starts), lo = __ffs(starts) - 1, hi = last + run_length(cont, last);
+  using elem_t = typename ElemOf<E>::type;
+  for (int base = lo; base < hi; base += 16) {
+    const int l = base + i;
+    const long long s = __shfl_sync(0xffffffffu, slot, min(l, 31));
+    if (l >= hi || s < 0) continue;
+    const uint8_t* row = value + (size_t)(first - 1 + l) * value_stride * E;
+    uint8_t* tile = vcache + ((size_t)(s / B) * kbs + (size_t)h0 * khs) * E + (s & (B - 1)) * E;
+    for (int c = g; c < nch; c += 8) {
+      uint4 v[kWinHeads];
+#pragma unroll
+      for (int k = 0; k < kWinHeads; ++k)
+        if (h0 + k < H) v[k] = __ldg(reinterpret_cast<const uint4*>(row + (size_t)(h0 + k) * D * E) + c);
+#pragma unroll
+      for (int k = 0; k < kWinHeads; ++k) {
+        if (h0 + k < H) {
+          const elem_t* e = reinterpret_cast<const elem_t*>(&v[k]);
+          uint8_t* out = tile + (size_t)k * khs * E + (size_t)c * 16 * B;
+#pragma unroll
+          for (int j = 0; j < kVec; ++j) *reinterpret_cast<elem_t*>(out + j * B * E) = e[j];
+        }
+      }
+    }
+  }
 }
 
 // dest[dest_idx[i]] = cache row at slot src_slots[i], block size 16: a CTA takes the runs of slots that
@@ -511,6 +716,20 @@ static int kv_run_launch(bool fill, void* key, void* value, void* kcache, void* 
   if (!aligned16(key) || !aligned16(value) || !aligned16(kcache) || !aligned16(vcache)) return PB_ERR_INVALID_ARG;
   if (ks % vec || vs % vec || kbs % vec || khs % vec) return PB_ERR_INVALID_ARG;
   if (T > 0x7fffffffll) return PB_ERR_INVALID_ARG;
+  if (fill && B == 16) {  // the engine's block size; the others take the warp per (run, head) below
+    const dim3 grid((unsigned)((T + 15) / 16), (unsigned)((H + win_heads(false) - 1) / win_heads(false)));
+    const long long* no_pos = nullptr;
+    const uint8_t* no_table = nullptr;
+    const cudaError_t err =
+        E == 2 ? launch_kernel(fill_window_kernel<__half, false>, grid, dim3(128), 0, s, true, (uint8_t*)nullptr, (uint8_t*)key,
+                               (const uint8_t*)value, (uint8_t*)kcache, (uint8_t*)vcache, slots, is64, no_pos, no_table, 0, 0ll,
+                               T, 0, H, D, 0ll, ks, vs, kbs, khs, num_blocks, 0)
+               : launch_kernel(fill_window_kernel<float, false>, grid, dim3(128), 0, s, true, (uint8_t*)nullptr, (uint8_t*)key,
+                               (const uint8_t*)value, (uint8_t*)kcache, (uint8_t*)vcache, slots, is64, no_pos, no_table, 0, 0ll,
+                               T, 0, H, D, 0ll, ks, vs, kbs, khs, num_blocks, 0);
+    if (err != cudaSuccess) { set_cuda_error(err); return PB_ERR_LAUNCH; }
+    return PB_OK;
+  }
   const size_t smem = (size_t)kFillWarps * B * D * E;
   // few tokens (decode): spread the heads over more CTAs; many tokens (prefill): at most four CTAs per token
   unsigned hgroups = (unsigned)((H + kFillWarps - 1) / kFillWarps);
@@ -539,6 +758,12 @@ static cudaError_t rotary_fill_launch_t(void* q, void* k, const void* v, void* k
                                         long long T_tok, int Hq, int H, int D, int B, long long qs, long long ks,
                                         long long vs, long long kbs, long long khs, long long num_blocks, int write_back,
                                         cudaStream_t s) {
+  if (B == 16) {  // the engine's block size (and rotation without a cache)
+    const dim3 win((unsigned)((T_tok + 15) / 16), (unsigned)(((Hq > H ? Hq : H) + win_heads(true) - 1) / win_heads(true)));
+    return launch_kernel(fill_window_kernel<T, true>, win, dim3(128), 0, s, true, (uint8_t*)q, (uint8_t*)k, (const uint8_t*)v,
+                         (uint8_t*)kc, (uint8_t*)vc, slots, is64, (const long long*)positions, (const uint8_t*)cos_sin, rot_dim,
+                         max_pos, T_tok, Hq, H, D, qs, ks, vs, kbs, khs, num_blocks, write_back);
+  }
   const size_t smem = (size_t)kFillWarps * B * D * sizeof(T);
   auto kfn = rotary_fill_kernel<T>;
   cudaError_t e = cudaSuccess;

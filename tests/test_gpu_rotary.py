@@ -116,6 +116,36 @@ def test_fused_rotary_fill_matches_rotary_then_fill(dtype, write_back):
         assert torch.equal(k, k0)
 
 
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("hq,hk,d,rot", [(6, 3, 128, 128), (3, 5, 128, 64), (5, 5, 64, 64), (2, 1, 256, 128), (4, 4, 80, 32)])
+@pytest.mark.parametrize("b", [8, 16])
+def test_fused_rotary_fill_over_head_counts_and_sizes(dtype, hq, hk, d, rot, b):
+    """Head counts that are no multiple of the heads a CTA takes, more query than kv heads and the reverse,
+    partly rotated rows; runs at odd offsets and lone tokens. (Block size 16 has a kernel of its own.)"""
+    nb, max_pos = 512 // b, 300
+    slots = np.asarray([s + i for s, n in [(5 * 16, 48), (9 * 16 + 7, 21), (20 * 16 + 15, 1), (21 * 16, 1), (33, 12), (300, 4)] for i in range(n)])
+    t = len(slots)
+    g = torch.Generator(device=DEV).manual_seed(11)
+    x = 16 // torch.empty((), dtype=dtype).element_size()
+    kc = torch.randn((nb, hk, d // x, b, x), generator=g, device=DEV).to(dtype)
+    vc = torch.randn((nb, hk, d, b), generator=g, device=DEV).to(dtype)
+    qkv = torch.randn((t, (hq + 2 * hk) * d), generator=g, device=DEV).to(dtype)
+    q, k, v = qkv.split([hq * d, hk * d, hk * d], dim=-1)
+    positions = torch.randint(0, max_pos, (t,), generator=g, device=DEV)
+    cs = cos_sin_table(max_pos, rot, dtype)
+    wq, wk = orc.rotary_neox_reference(positions.cpu().numpy(), q.cpu().double().numpy(), k.cpu().double().numpy(),
+                                       cs.cpu().double().numpy(), d)
+    kr, vr = bits(kc).copy(), bits(vc).copy()
+    pb.rotary_reshape_and_cache(positions, q, k, v, kc, vc, torch.tensor(slots, device=DEV), cs, d)
+    assert_rotated(q, wq, dtype, "query")
+    k_back, v_back = (torch.zeros((t, hk, d), dtype=dtype, device=DEV) for _ in range(2))
+    pb.gather_cached_kv(k_back, v_back, kc, vc, torch.tensor(slots, device=DEV))
+    assert_rotated(k_back.view(t, -1), wk, dtype, "cached key")
+    assert np.array_equal(bits(v_back.view(t, -1)), bits(v))
+    orc.fill_reference(bits(k_back), bits(v_back), kr, vr, slots)  # nothing but the addressed slots changed
+    assert np.array_equal(bits(kc), kr) and np.array_equal(bits(vc), vr)
+
+
 def test_rotary_rejects_unsupported_shapes():
     q = torch.zeros((2, 128), dtype=torch.float16, device=DEV)
     cs = torch.zeros((8, 24), dtype=torch.float16, device=DEV)  # halves of 12 elements: not whole 16-byte chunks
