@@ -201,6 +201,38 @@ def test_several_query_heads_per_item(dtype, kv, share, d, usual):
     assert_close_to_oracle(out, ref, dtype, f"{share} query heads per kv head, head size {d}")
 
 
+@pytest.mark.parametrize("rows", [1, 1023, 1025, 4096, 4097])
+def test_work_lists_over_row_counts(rows):
+    """Rows without a suffix at the start, in the middle and at the end, rows of one and of several chunks, around
+    the row counts at which the planner changes how it writes the items; with the rows' new tokens in the call."""
+    rng = np.random.default_rng(rows)
+    sl = np.where(rng.random(rows) < 0.2, 0, rng.integers(1, 200, size=rows))
+    sl[[0, -1]] = 0 if rows > 1 else 37
+    nb = int(((sl + 15) // 16).sum()) + 1
+    g = torch.Generator(device=DEV).manual_seed(90)
+    kc, vc = torch.randn((nb, 1, 16, 16, 8), generator=g, device=DEV).half(), torch.randn((nb, 1, 128, 16), generator=g, device=DEV).half()
+    q, k, v = (torch.randn((rows, 1, 128), generator=g, device=DEV).half() for _ in range(3))
+    perm, at, st = rng.permutation(nb), 0, np.zeros((rows, 13), dtype=np.int32)
+    for r in range(rows):
+        n = (sl[r] + 15) // 16
+        st[r, :n] = perm[at:at + n]
+        at += n
+    slots = np.where(sl > 0, st[np.arange(rows), np.maximum(sl - 1, 0) // 16].astype(np.int64) * 16 + (sl - 1) % 16, -1)
+    call = pb.AttentionCall(num_rows=rows, num_heads=1, head_size=128, block_size=16, dtype=torch.float16, device=q.device,
+                            suffix_lens=torch.tensor(sl, dtype=torch.int32, device=DEV), suffix_tables=torch.tensor(st, device=DEV),
+                            slot_mapping=torch.tensor(slots, device=DEV), suffix_chunk_blocks=4)
+    kr, vr = kc.cpu().numpy().view(np.int16).copy(), vc.cpu().numpy().view(np.int16).copy()
+    out = torch.empty_like(q)
+    call.plan(q, out, kc, vc)
+    call.run(q, out, kc, vc, key_new=k, value_new=v)
+    assert call.status() == 0
+    orc.fill_reference(k.cpu().numpy().view(np.int16), v.cpu().numpy().view(np.int16), kr, vr, slots)
+    assert np.array_equal(kc.cpu().numpy().view(np.int16), kr) and np.array_equal(vc.cpu().numpy().view(np.int16), vr)
+    some = sorted(set(range(0, rows, 17)) | {rows - 1})
+    ref = orc.gold_grouped_attention(q.float().cpu(), kc.float().cpu(), vc.float().cpu(), None, None, None, sl.tolist(), st.tolist(), rows=some)
+    assert_close_to_oracle(out[some], ref, torch.float16, f"{rows} rows")
+
+
 def test_prev_post_native_entry_points():
     """prev writes normalised out + base-2 stats; post merges a second context into it in place:
     prev(A) then post(B) == attention over A ++ B (csrc/attention.cpp:19-47)."""
