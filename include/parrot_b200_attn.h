@@ -401,6 +401,12 @@ int pb_sample_top_p(const void* logits, int32_t dtype, int32_t num_rows, int32_t
                     const float* temperature, const float* top_p, const float* uniforms, int64_t* ids,
                     void* stream);
 
+/* The same with the rows' settings in HOST memory (num_rows floats each, NULL = 1.0 for every row): they
+ * are passed to the kernel by value, so that nothing is uploaded and the arrays may be reused at once. */
+int pb_sample_top_p_host_settings(const void* logits, int32_t dtype, int32_t num_rows, int32_t vocab, int64_t row_stride,
+                                  const float* h_temperature, const float* h_top_p, const float* uniforms, int64_t* ids,
+                                  void* stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -252,7 +252,8 @@ _staging = {}  # device index -> [page-locked buffer, event of the last upload f
 def _upload_packed(arrays: dict, dev: torch.device) -> dict:
     """All index arrays of an iteration in ONE host-to-device transfer from a reused page-locked
     buffer (a dozen separate small pageable uploads cost more than the attention of a layer);
-    returns device tensors (views of one allocation) under the same names."""
+    returns device tensors (views of one allocation) under the same names. The arrays are int32 or
+    int64, of one or two dimensions."""
     if dev.type != "cuda":
         return {n: torch.from_numpy(np.ascontiguousarray(a)).to(dev) for n, a in arrays.items()}
     offs, total = {}, 0
@@ -272,9 +273,13 @@ def _upload_packed(arrays: dict, dev: torch.device) -> dict:
     d[:total].copy_(st[0][:total], non_blocking=True)
     st[1] = torch.cuda.Event()
     st[1].record(torch.cuda.current_stream(dev))
+    # one view per array: of the buffer as a whole in the array's type, placed by its offset
+    as_type = {4: d.view(torch.int32), 8: d.view(torch.int64)}
     out = {}
     for n, a in arrays.items():
-        out[n] = d[offs[n]:offs[n] + a.nbytes].view(torch.from_numpy(np.empty(0, dtype=a.dtype)).dtype).view(a.shape)
+        width = a.itemsize
+        strides = (1,) if a.ndim == 1 else (a.shape[1], 1)
+        out[n] = as_type[width].as_strided(a.shape, strides, offs[n] // width)
     return out
 
 
@@ -388,8 +393,10 @@ class B200SharedPromptsGenerate(nn.Module):
                 iteration_state.b200_planned = True
             call.params.scale = float(self.scaling)
             if fused:  # KV fill and attention as one call
-                call.run(q, output, k_cache, v_cache, key_new=k.view(q.shape[0], -1, self.head_dim),
-                         value_new=v.view(q.shape[0], -1, self.head_dim))
+                d = self.head_dim
+                if k.dim() != 3 or k.shape[2] != d or v.dim() != 3 or v.shape[2] != d:
+                    k, v = k.view(q.shape[0], -1, d), v.view(q.shape[0], -1, d)
+                call.run(q, output, k_cache, v_cache, key_new=k, value_new=v)
             else:
                 call.run(q, output, k_cache, v_cache)
         return output.view(-1, self.num_heads * self.head_dim)

@@ -181,16 +181,31 @@ __device__ __forceinline__ void refine_add(SampShared& sh, float d, int level, u
   if (q) hist_add(sh, (int)((key >> shift) & (kBins - 1)), q);  // weightless tokens change no sum
 }
 
-template <typename T>
+// Settings of up to kSettingsRows rows that the caller has on the host: they travel as a kernel parameter (an
+// upload of each list was two synchronous copies, together longer than the kernel).
+constexpr int kSettingsRows = 256;
+struct SampSettings {
+  float temperature[kSettingsRows], top_p[kSettingsRows];
+};
+struct NoSettings {};
+
+template <typename T, typename Settings>
 __global__ void __launch_bounds__(kSampThreads) sample_top_p_kernel(
     const T* __restrict__ logits, const int vocab, const long long row_stride, const float* __restrict__ temperature,
-    const float* __restrict__ top_p, const float* __restrict__ uniforms, long long* __restrict__ ids) {
+    const float* __restrict__ top_p, const __grid_constant__ Settings settings, const float* __restrict__ uniforms,
+    long long* __restrict__ ids) {
   __shared__ SampShared sh;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const T* row = logits + (long long)blockIdx.x * row_stride;
   const bool vec = (reinterpret_cast<uintptr_t>(row) & 15) == 0;
-  const float temp = temperature ? __fdiv_rn(1.f, temperature[blockIdx.x]) : 1.f;  // 1 / temperature
-  const float p_keep = top_p ? fmaxf(top_p[blockIdx.x], 0.f) : 1.f;
+  float temp = 1.f, p_keep = 1.f;  // temp: 1 / temperature
+  if constexpr (sizeof(Settings) > sizeof(NoSettings)) {
+    temp = __fdiv_rn(1.f, settings.temperature[blockIdx.x]);
+    p_keep = fmaxf(settings.top_p[blockIdx.x], 0.f);
+  } else {
+    if (temperature) temp = __fdiv_rn(1.f, temperature[blockIdx.x]);
+    if (top_p) p_keep = fmaxf(top_p[blockIdx.x], 0.f);
+  }
 
   // Every pass walks the row in tiles of kTile tokens; the next tile's loads are issued before the
   // current tile is processed.
@@ -384,6 +399,26 @@ __global__ void __launch_bounds__(kSampThreads) sample_top_p_kernel(
   if (tid == 0) ids[blockIdx.x] = sh.found == 0x7fffffff ? (long long)(vocab - 1) : (long long)sh.found;
 }
 
+
+template <typename Settings>
+int launch_sample(const void* logits, int32_t dtype, int32_t rows, int32_t vocab, int64_t row_stride, const float* temperature,
+                  const float* top_p, const Settings& settings, const float* uniforms, int64_t* ids, cudaStream_t s) {
+  long long* out = reinterpret_cast<long long*>(ids);
+#define PB_SAMPLE(TT)                                                                                          \
+  sample_top_p_kernel<TT, Settings><<<rows, kSampThreads, 0, s>>>(static_cast<const TT*>(logits), vocab, row_stride, \
+                                                                  temperature, top_p, settings, uniforms, out)
+  switch (dtype) {
+    case PB_F32: PB_SAMPLE(float); break;
+    case PB_F16: PB_SAMPLE(__half); break;
+    case PB_BF16: PB_SAMPLE(__nv_bfloat16); break;
+    default: return PB_ERR_UNSUPPORTED;
+  }
+#undef PB_SAMPLE
+  const cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) { set_cuda_error(e); return PB_ERR_LAUNCH; }
+  return PB_OK;
+}
+
 }  // namespace
 }  // namespace pb
 
@@ -393,25 +428,28 @@ extern "C" int pb_sample_top_p(const void* logits, int32_t dtype, int32_t num_ro
   if (num_rows < 0 || vocab <= 0 || row_stride < vocab) return PB_ERR_INVALID_ARG;
   if (num_rows == 0) return PB_OK;
   if (!logits || !uniforms || !ids) return PB_ERR_INVALID_ARG;
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
-  long long* out = reinterpret_cast<long long*>(ids);
-  switch (dtype) {
-    case PB_F32:
-      pb::sample_top_p_kernel<float><<<num_rows, pb::kSampThreads, 0, s>>>(
-          static_cast<const float*>(logits), vocab, row_stride, temperature, top_p, uniforms, out);
-      break;
-    case PB_F16:
-      pb::sample_top_p_kernel<__half><<<num_rows, pb::kSampThreads, 0, s>>>(
-          static_cast<const __half*>(logits), vocab, row_stride, temperature, top_p, uniforms, out);
-      break;
-    case PB_BF16:
-      pb::sample_top_p_kernel<__nv_bfloat16><<<num_rows, pb::kSampThreads, 0, s>>>(
-          static_cast<const __nv_bfloat16*>(logits), vocab, row_stride, temperature, top_p, uniforms, out);
-      break;
-    default:
-      return PB_ERR_UNSUPPORTED;
+  return pb::launch_sample(logits, dtype, num_rows, vocab, row_stride, temperature, top_p, pb::NoSettings{}, uniforms, ids,
+                           static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int pb_sample_top_p_host_settings(const void* logits, int32_t dtype, int32_t num_rows, int32_t vocab,
+                                             int64_t row_stride, const float* h_temperature, const float* h_top_p,
+                                             const float* uniforms, int64_t* ids, void* stream) {
+  if (num_rows < 0 || vocab <= 0 || row_stride < vocab) return PB_ERR_INVALID_ARG;
+  if (num_rows == 0) return PB_OK;
+  if (!logits || !uniforms || !ids) return PB_ERR_INVALID_ARG;
+  if (dtype != PB_F32 && dtype != PB_F16 && dtype != PB_BF16) return PB_ERR_UNSUPPORTED;
+  const size_t row_bytes = (size_t)row_stride * (dtype == PB_F32 ? 4 : 2);
+  for (int32_t r0 = 0; r0 < num_rows; r0 += pb::kSettingsRows) {
+    const int32_t n = num_rows - r0 < pb::kSettingsRows ? num_rows - r0 : pb::kSettingsRows;
+    pb::SampSettings set;
+    for (int32_t i = 0; i < pb::kSettingsRows; ++i) {
+      set.temperature[i] = (h_temperature && i < n) ? h_temperature[r0 + i] : 1.f;
+      set.top_p[i] = (h_top_p && i < n) ? h_top_p[r0 + i] : 1.f;
+    }
+    const int rc = pb::launch_sample(static_cast<const char*>(logits) + r0 * row_bytes, dtype, n, vocab, row_stride, nullptr,
+                                     nullptr, set, uniforms + r0, ids + r0, static_cast<cudaStream_t>(stream));
+    if (rc != PB_OK) return rc;
   }
-  const cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) { pb::set_cuda_error(e); return PB_ERR_LAUNCH; }
   return PB_OK;
 }

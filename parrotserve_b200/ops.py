@@ -38,7 +38,8 @@ def _require_cuda(*tensors: torch.Tensor) -> None:
 
 
 def _stream(t: torch.Tensor) -> int:
-    return torch.cuda.current_stream(t.device).cuda_stream
+    # the raw handle of torch.cuda.current_stream(t.device), without building a Stream object per call
+    return torch._C._cuda_getCurrentRawStream(t.get_device())
 
 
 def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
@@ -71,16 +72,19 @@ def _kv_geometry(key_cache: torch.Tensor, value_cache: torch.Tensor):
     if key_cache.dim() != 5 or value_cache.dim() != 4:
         raise RuntimeError("key_cache must be [NB,H,D/x,B,x] and value_cache [NB,H,D,B]")
     nb, hkv, d, b = value_cache.shape
-    x = key_cache.shape[4]
-    if key_cache.shape[0] != nb or key_cache.shape[1] != hkv or key_cache.shape[2] * x != d or key_cache.shape[3] != b:
+    knb, khkv, kdx, kb, x = key_cache.shape
+    if knb != nb or khkv != hkv or kdx * x != d or kb != b:
         raise RuntimeError("key_cache / value_cache shapes disagree")
     if x * key_cache.element_size() != 16:
         raise RuntimeError("key_cache innermost dimension must span 16 bytes")
-    if key_cache.stride(0) != value_cache.stride(0) or key_cache.stride(1) != value_cache.stride(1):
+    ks, vs = key_cache.stride(), value_cache.stride()
+    if ks[0] != vs[0] or ks[1] != vs[1]:
         raise RuntimeError("key_cache and value_cache must share block and head strides")
-    if key_cache[0, 0].is_contiguous() is False or value_cache[0, 0].is_contiguous() is False:
-        raise RuntimeError("a (block, head) tile must be contiguous")
-    return nb, hkv, d, b, key_cache.stride(0), key_cache.stride(1)
+    # the usual strides of a tile are compared as they are; others (dimensions of size one, empty caches) by building its view
+    if not (nb and hkv and ks[2:] == (b * x, x, 1) and vs[2:] == (b, 1)):
+        if key_cache[0, 0].is_contiguous() is False or value_cache[0, 0].is_contiguous() is False:
+            raise RuntimeError("a (block, head) tile must be contiguous")
+    return nb, hkv, d, b, ks[0], ks[1]
 
 
 class AttentionCall:
@@ -234,30 +238,22 @@ class AttentionCall:
         p.workspace = self.workspace.data_ptr()
         p.workspace_bytes = self.workspace.numel()
         self._planned = False
-        self._bound = {}
+        self._params_ref = C.byref(p)
+        self._q_shape = (num_rows, num_heads, head_size)
 
     def _bind(self, query, out, key_cache, value_cache, qk_max=None, exp_sum=None, stats_mode=_lib.PB_STATS_NONE):
         p = self.params
-        # the same tensors as in an earlier call (every layer of an iteration, every step of a loop):
-        # their checks and geometry are remembered, only the pointers are rewritten
-        key = (query.data_ptr(), out.data_ptr(), key_cache.data_ptr(), value_cache.data_ptr(), query.stride(0), out.stride(0),
-               query.shape, out.shape, key_cache.shape, query.dtype, out.dtype, key_cache.dtype)
-        hit = self._bound.get(key)
-        if hit is not None and stats_mode == _lib.PB_STATS_NONE:
-            (p.out, p.query, p.key_cache, p.value_cache, p.num_kv_heads, p.num_blocks, p.q_stride, p.out_stride,
-             p.kv_block_stride, p.kv_head_stride) = hit
-            p.qk_max = p.exp_sum = None
-            p.stats_mode = stats_mode
-            return
         _require_cuda(query, out, key_cache, value_cache)
         nb, hkv, d, b, kbs, khs = _kv_geometry(key_cache, value_cache)
-        if query.dtype != self.dtype or key_cache.dtype != self.dtype or value_cache.dtype != self.dtype or out.dtype != self.dtype:
+        dtype = self.dtype
+        if query.dtype != dtype or key_cache.dtype != dtype or value_cache.dtype != dtype or out.dtype != dtype:
             raise RuntimeError("query, caches and out must share the dtype of the call")
-        if query.dim() != 3 or query.shape[0] != p.num_rows or query.shape[1] != p.num_heads or query.shape[2] != p.head_size:
+        if query.shape != self._q_shape:
             raise RuntimeError(f"query must be [{p.num_rows}, {p.num_heads}, {p.head_size}]")
-        if d != p.head_size or b != p.block_size:
+        if d != self._q_shape[2] or b != p.block_size:
             raise RuntimeError("cache head_size/block_size differ from the call's")
-        if query.stride(2) != 1 or query.stride(1) != d or out.stride(2) != 1 or out.stride(1) != d:
+        qs, os = query.stride(), out.stride()
+        if qs[2] != 1 or qs[1] != d or os[2] != 1 or os[1] != d:
             raise RuntimeError("query/out must be dense over (head, dim)")
         p.out = out.data_ptr()
         p.query = query.data_ptr()
@@ -265,19 +261,13 @@ class AttentionCall:
         p.value_cache = value_cache.data_ptr()
         p.num_kv_heads = hkv
         p.num_blocks = nb
-        p.q_stride = query.stride(0)
-        p.out_stride = out.stride(0)
+        p.q_stride = qs[0]
+        p.out_stride = os[0]
         p.kv_block_stride = kbs
         p.kv_head_stride = khs
         p.qk_max = _ptr(qk_max)
         p.exp_sum = _ptr(exp_sum)
         p.stats_mode = stats_mode
-        if len(self._bound) > 64:
-            self._bound.clear()
-        # (shapes and dtypes were checked above; a tensor freed and another allocated at the same
-        # address with other strides gets a different key through the strides)
-        self._bound[key] = (p.out, p.query, p.key_cache, p.value_cache, p.num_kv_heads, p.num_blocks, p.q_stride,
-                            p.out_stride, p.kv_block_stride, p.kv_head_stride)
 
     def plan(self, query, out, key_cache, value_cache) -> None:
         self._bind(query, out, key_cache, value_cache)
@@ -295,19 +285,20 @@ class AttentionCall:
             if not self._has_slots:
                 raise RuntimeError("key_new / value_new need the slot_mapping given to AttentionCall")
             _require_cuda(key_new, value_new)
-            shape = (p.num_rows, p.num_kv_heads, p.head_size)
-            for x in (key_new, value_new):
-                if tuple(x.shape) != shape or x.dtype != self.dtype or x.stride(2) != 1 or x.stride(1) != p.head_size:
-                    raise RuntimeError(f"key_new / value_new must be {shape}, dense over (head, dim), of the call's dtype")
+            rows, _, d = self._q_shape
+            shape = (rows, p.num_kv_heads, d)
+            ks, vs = key_new.stride(), value_new.stride()
+            if (key_new.shape != shape or value_new.shape != shape or key_new.dtype != self.dtype or value_new.dtype != self.dtype
+                    or ks[1:] != (d, 1) or vs[1:] != (d, 1)):
+                raise RuntimeError(f"key_new / value_new must be {shape}, dense over (head, dim), of the call's dtype")
             p.key_new, p.value_new = key_new.data_ptr(), value_new.data_ptr()
-            p.key_new_stride, p.value_new_stride = key_new.stride(0), value_new.stride(0)
+            p.key_new_stride, p.value_new_stride = ks[0], vs[0]
         else:
             p.key_new = p.value_new = None
-        if self._planned:
-            rc = lib().pb_shared_prefix_attention_planned(C.byref(self.params), _stream(query))
-        else:
-            rc = lib().pb_shared_prefix_attention(C.byref(self.params), _stream(query))
-        check(rc, "pb_shared_prefix_attention")
+        fn = lib().pb_shared_prefix_attention_planned if self._planned else lib().pb_shared_prefix_attention
+        rc = fn(self._params_ref, _stream(query))
+        if rc != _lib.PB_OK:
+            check(rc, "pb_shared_prefix_attention")
         return out
 
     def status(self) -> int:
@@ -847,7 +838,10 @@ def sample_top_p(logits: torch.Tensor, temperature=None, top_p=None, uniforms: O
                 raise ValueError("temperature must be positive")
             if all(t == 1.0 for t in v):
                 return None
-            v = torch.tensor(v, dtype=torch.float32, device=dev)
+            v = torch.tensor(v, dtype=torch.float32)  # on the host: handed to the kernel by value
+            if v.shape != (rows,):
+                raise RuntimeError(f"{name} must hold one number per row")
+            return v
         if v.shape != (rows,) or v.dtype != torch.float32 or v.device != dev or not v.is_contiguous():
             raise RuntimeError(f"{name} must be a contiguous float32 tensor [rows] on the logits' device")
         return v
@@ -856,12 +850,16 @@ def sample_top_p(logits: torch.Tensor, temperature=None, top_p=None, uniforms: O
     if uniforms is None:
         uniforms = torch.rand(rows, dtype=torch.float32, device=dev, generator=generator)
     uniforms = per_row(uniforms, "uniforms")
+    if uniforms is not None and not uniforms.is_cuda:
+        uniforms = uniforms.to(dev)
     ids = torch.empty(rows, dtype=torch.int64, device=dev)
     if rows == 0:
         return ids
-    rc = lib().pb_sample_top_p(logits.data_ptr(), _dtype_code(logits), rows, vocab, logits.stride(0),
-                               temperature.data_ptr() if temperature is not None else None,
-                               top_p.data_ptr() if top_p is not None else None,
-                               uniforms.data_ptr(), ids.data_ptr(), _stream(logits))
+    on_host = [v is None or not v.is_cuda for v in (temperature, top_p)]
+    if not all(on_host):  # one of them a device tensor: both in device memory
+        temperature, top_p = (v.to(dev) if v is not None and not v.is_cuda else v for v in (temperature, top_p))
+    fn = lib().pb_sample_top_p_host_settings if all(on_host) else lib().pb_sample_top_p
+    rc = fn(logits.data_ptr(), _dtype_code(logits), rows, vocab, logits.stride(0), _ptr(temperature), _ptr(top_p),
+            uniforms.data_ptr(), ids.data_ptr(), _stream(logits))
     check(rc, "pb_sample_top_p")
     return ids

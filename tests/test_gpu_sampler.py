@@ -199,6 +199,26 @@ def test_sampler_module_has_the_reference_interface():
         ops.sample_top_p(logits, [0.0] * 5, None, u)
 
 
+@pytest.mark.parametrize("rows", [1, 255, 256, 257, 600])
+def test_settings_on_the_host_draw_what_settings_on_the_device_draw(rows):
+    """Settings given as numbers travel by value, 256 rows to a launch; as tensors they are read from memory."""
+    g = torch.Generator(device=DEV).manual_seed(rows)
+    logits = torch.randn((rows, 1000), generator=g, device=DEV) * 3
+    u = torch.rand(rows, generator=g, device=DEV)
+    rng = np.random.default_rng(rows)
+    temperature = rng.uniform(0.5, 1.5, rows).astype(np.float32).tolist()
+    top_p = np.where(rng.random(rows) < 0.3, 1.0, rng.uniform(0.1, 0.99, rows)).astype(np.float32).tolist()
+    dt, dp = (torch.tensor(v, dtype=torch.float32, device=DEV) for v in (temperature, top_p))
+    want = ops.sample_top_p(logits, dt, dp, uniforms=u)
+    assert torch.equal(ops.sample_top_p(logits, temperature, top_p, uniforms=u), want)
+    assert torch.equal(ops.sample_top_p(logits, temperature, dp, uniforms=u), want)  # one of each
+    want = ops.sample_top_p(logits, None, dp, uniforms=u)
+    assert torch.equal(ops.sample_top_p(logits, None, top_p, uniforms=u), want)
+    assert torch.equal(ops.sample_top_p(logits, [1.0] * rows, top_p, uniforms=u), want)
+    with pytest.raises(RuntimeError):
+        ops.sample_top_p(logits, temperature + [0.7], top_p, uniforms=u)
+
+
 def test_c_entry_rejects_bad_arguments():
     from parrotserve_b200 import _lib
 
