@@ -18,7 +18,7 @@ constexpr int kPairLanes = 16;                 // lanes that share one (row, hea
 constexpr int kPairsPerWarp = 32 / kPairLanes;  // two (row, head) pairs per warp: twice the loads in flight
 constexpr int kPairs = kMergeWarps * kPairsPerWarp;  // heads a CTA works on at once
 constexpr int kMaxHeadsPerCta = kMergeWarps * 32;    // one thread each finds a head's partials
-constexpr int kManyRows = 1024;                      // from here on one CTA takes up to kMaxHeadsPerCta heads of a row
+constexpr int kManyRows = 1024;                      // prefill batches from here on: a CTA takes up to kMaxHeadsPerCta heads of a row
 
 // dense_cta_of_tile, with a 32-bit division wherever the product fits: the 64-bit one is a routine of some
 // hundred instructions, and every (row, head) asks twice.
@@ -210,7 +210,7 @@ __global__ void __launch_bounds__(kMergeWarps * 32) merge_kernel(const AttnDev d
 
 template <typename T, int D>
 cudaError_t launch_merge_d(const AttnDev& d, cudaStream_t s) {
-  const bool many = d.num_rows >= kManyRows;
+  const bool many = d.num_segments > 0 && d.num_rows >= kManyRows;  // (only prefill rows are ever finished before)
   const int hpc = !many ? kPairs : d.num_heads < kMaxHeadsPerCta ? d.num_heads : kMaxHeadsPerCta;
   const unsigned grid = (unsigned)((long long)d.num_rows * ((d.num_heads + hpc - 1) / hpc));
   return many ? launch_kernel(merge_kernel<T, D, true>, grid, kMergeWarps * 32, (size_t)hpc * sizeof(int4), s, true, d, hpc)
