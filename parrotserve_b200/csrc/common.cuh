@@ -87,10 +87,11 @@ constexpr int32_t kDnDirect = 1;
 // What one (item, head) costs beside its kv tiles, in tiles: the load of Q, the first tile's way through the
 // pipeline, the epilogue. Causal items have from one kv tile to dozens, so CTAs with equal shares of the
 // tiles alone had very unequal work (those with the short row tiles of a prefill up to ten times as many
-// epilogues, and the SMs were busy 54 % of the kernel's time). Four prompts of 1500..3000 tokens: 645 us with
-// 0, 483 with 2, 485 with 3, 488 with 5; 16 prefills under a shared prefix are indifferent to 2 (1226).
+// epilogues, and the SMs were busy 54 % of the kernel's time). Four prompts of 1500..3000 tokens, single row
+// tiles: 645 us with 0, 483 with 2, 485 with 3, 488 with 5; row-tile pairs: 426 with 2, 417 with 3, 422 with 4; 16
+// prefills under a shared prefix are indifferent (1135, 1134, 1132).
 // Items without a causal mask are equally long within a group; their tiles are split as they are.
-constexpr int32_t kCausalFixedTiles = 2;
+constexpr int32_t kCausalFixedTiles = 3;
 constexpr int32_t kDnOuter = 2;   // the item walks an outer prefix group (outer_tables, outer partial range)
 
 struct WsLayout {

@@ -7,7 +7,7 @@
 // Q.K^T of one tile, the softmax threads of the other tile are at work. (They used to take turns at the
 // exponentials, one warp per scheduler at a time; one warp alone keeps the special-function unit little more
 // than half busy, two reach its rate of 8 cycles per instruction: four prompts of 1500..3000 tokens took
-// 477 us with turns and 434 us without.) Per row tile x (0, 1):
+// 477 us with those turns and 434 us without. The issue of the MMAs takes turns instead.) Per row tile x (0, 1):
 //     S_x[128 x 128] = Q_x . K^T         (A and B from shared memory)
 //     O_x[128 x D]  += P_x . V           (A = P_x from TENSOR MEMORY, B from shared memory)
 // Tensor memory (512 columns): S_0 [0,128), S_1 [128,256), O_0 [256,384), O_1 [384,512). P_x is
@@ -53,7 +53,8 @@ enum {
   kBarQFree = 16,    // every Q_x.K^T of a segment has retired: Q_x may be overwritten
   kBarODrained = 18, // the epilogue of a segment has read O_x out of tensor memory
   kBarGroup = 20,    // meeting point of the 128 softmax threads of row tile x (bounded, unlike bar.sync)
-  kNumBars = 22
+  kBarTurn = 22,     // issuer x has issued P_x.V and the next Q_x.K^T of a kv tile (pair items)
+  kNumBars = 24
 };
 
 
@@ -187,6 +188,7 @@ dense_pair_kernel(const AttnDev d, const __grid_constant__ CUtensorMap vmap, con
       mbar_init(bar(kBarQ + x), 1);
       mbar_init(bar(kBarQFree + x), 1);
       mbar_init(bar(kBarODrained + x), kGroupThreads);
+      mbar_init(bar(kBarTurn + x), 1);
       mbar_init(bar(kBarGroup + x), kGroupThreads);
     }
     *abort_flag = 0;
@@ -250,7 +252,10 @@ dense_pair_kernel(const AttnDev d, const __grid_constant__ CUtensorMap vmap, con
     //                  thread's program order, which the tensor pipe keeps
     // Two issuers, one per row tile: their chains are independent (disjoint tensor memory) and the
     // instruction stream of one thread cannot feed the pipe for both. A K (V) slot is released by
-    // the second of the two commits on it.
+    // the second of the two commits on it. On pair items they issue in turns (0, 1, 0, 1, ...): issued
+    // together, the MMAs of both tiles share the pipe and end together, and the two softmax groups fall into
+    // step, both at the exponentials, then both waiting. 16 prefills of 256..1024 tokens with 240 decodes under a
+    // 2048-token prefix: 1203 -> 1132 us; four prompts of 1500..3000 tokens unchanged (415, with 3 fixed tiles).
     // The operand descriptors are built once; an MMA adds its offset to the address field. (Built per
     // MMA, the descriptor arithmetic of the issuing thread costs more than the MMA itself.)
     //   Q_x: [64-element half][row][128 B], 128-byte swizzle -> SBO 1024 (8-row groups)
@@ -263,10 +268,11 @@ dense_pair_kernel(const AttnDev d, const __grid_constant__ CUtensorMap vmap, con
     const uint64_t desc_k0 = smem_desc(sK0, 2048, 128, 0), desc_k1 = smem_desc(sK0 + kRingBytes, 2048, 128, 0);
     const uint64_t desc_v0 = smem_desc(sV0, 16, 256, 6), desc_v1 = smem_desc(sV0 + kRingBytes, 16, 256, 6);
     const uint32_t tmem_s = tmem_base + x * 128, tmem_o = tmem_base + 256 + x * 128;
-    uint32_t tc = 0, tcx = 0, segx = 0;
+    uint32_t tc = 0, tcx = 0, segx = 0, turns = 0;  // turns: kv tiles of pair items so far
     bool ok = true;
     while (ok && walk.next(sg)) {
       const int n = sg.t1 - sg.t0;
+      const bool pair = sg.it.nrows > 128;
       if (x == 1 && sg.it.nrows <= 128) {
         // a lone row tile: nothing to compute here, but every ring slot still takes this issuer's release
         for (int i = 0; i < n && ok; ++i, ++tc) {
@@ -313,6 +319,8 @@ dense_pair_kernel(const AttnDev d, const __grid_constant__ CUtensorMap vmap, con
         if (i == 0 && segx > 0 && !wait_or_abort(bar(kBarODrained + x), (segx - 1) & 1, abort_flag, status)) { ok = false; break; }
         fence_proxy_async_smem();
         if (!wait_or_abort(bar(kBarP + x), (tcx + i) & 1, abort_flag, status)) { ok = false; break; }
+        if (pair && (x == 1 || turns > 0) &&
+            !wait_or_abort(bar(kBarTurn + (x ^ 1)), (x == 1 ? turns : turns - 1) & 1, abort_flag, status)) { ok = false; break; }
         tc_fence_after();
         if (lane == 0) {
           PB_TRACE(30 + x);
@@ -322,12 +330,14 @@ dense_pair_kernel(const AttnDev d, const __grid_constant__ CUtensorMap vmap, con
           for (int j = 0; j < kTileBlocks; ++j)
             if (j < nb) mma_f16_ts(tmem_o, tmem_s + j * 8, bv + j * (kBlkBytes >> 4), kIdescPV, (i > 0 || j > 0) ? 1u : 0u);
           if (more) qk_mmas(i + 1);  // behind P_x.V(i) in the pipe: it overwrites S_x / P_x
+          if (pair) mbar_arrive(bar(kBarTurn + x));
           PB_TRACE(32 + x);
           mma_commit(bar(kBarPV + x));
           mma_commit(bar(kBarEmptyV + s));
           if (more) qk_release(i + 1);
           PB_TRACE(20 + x);
         }
+        if (pair) ++turns;
         __syncwarp();
       }
       if (!ok) break;
