@@ -123,10 +123,8 @@ __global__ void __launch_bounds__(kMergeWarps * 32) merge_kernel(const AttnDev d
   for (int j = sub + kPairLanes; j < n; j += kPairLanes) M = fmaxf(M, d.ml[partial_slot(d, row, part_of(j), head)].x);
 #pragma unroll
   for (int o = kPairLanes / 2; o >= 1; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
-  // Everything this kernel reads of the planner's output has arrived (the statistics just reduced
-  // were addressed with it), so the next kernel in the stream may become resident: an attention
-  // kernel or a KV fill waits for this grid's completion before it touches anything, and a planner
-  // only overwrites the lists read above and completes after this grid.
+  // The next kernel in the stream may become resident: every kernel of this library that is launched early
+  // waits for this grid's completion before it writes anything to global memory (the planner counts first).
   if (hb == h_lo) pdl_trigger();
 
   float4 o4[kPer];

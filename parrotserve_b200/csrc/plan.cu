@@ -212,14 +212,18 @@ __global__ void __launch_bounds__(kPlanThreads, 1) plan_kernel(const AttnDev d, 
   constexpr int kCarries = 1 << 30;
   __shared__ int row_first[kFlatRows + 1];
   __shared__ unsigned long long sq_blocks;  // blocks all single-query items stream, per head
+  // The kernel before this one may still be at work, and it may own the very memory this call's workspace lies
+  // in: a merge of another call on the same scratch, whose partials are where this call's lists go, or the
+  // stores of an output whose memory has been handed out again. Until pdl_wait() only lengths and offsets are read and nothing
+  // is written outside shared memory; faults found while counting are kept here.
+  __shared__ int32_t count_hdr[kHdrStatus + 1];
+  AttnDev c = d;
+  c.hdr = count_hdr;
   const int tid = threadIdx.x;
   const int S = d.num_rows, G = d.num_groups, NS = d.num_segments;
   const int RT = d.dense_row_tile;  // rows per dense item: 128, or 256 when the dense kernel works on row-tile pairs
 
-  if (tid == 0) {
-    d.hdr[kHdrStatus] = kStatusOk; d.hdr[kHdrSqCounter] = 0; sq_blocks = 0;
-    d.hdr[kHdrPlannedSlots] = (d.slot_mapping && NS == 0 && !d.head_mapping) ? 1 : 0;
-  }
+  if (tid == 0) { count_hdr[kHdrStatus] = kStatusOk; sq_blocks = 0; }
   __syncthreads();
 
   // ---- counts: groups (dense items / single-query prefix items) ----
@@ -228,9 +232,9 @@ __global__ void __launch_bounds__(kPlanThreads, 1) plan_kernel(const AttnDev d, 
   int my_dng = 0, my_dns = 0, my_sq = 0, my_tiles_g = 0, my_tiles_s = 0;
   long long my_blocks = 0;
   for (int g = g_lo; g < g_hi; ++g) {
-    const GroupPlan p = group_plan(d, g, B, dense_ok);
+    const GroupPlan p = group_plan(c, g, B, dense_ok);
     if (p.dense) {
-      walk_group_rows(d, g, p, B, dense_ok,
+      walk_group_rows(c, g, p, B, dense_ok,
                       [&](int r_lo, int r_hi) {
                         const int n_rt = (r_hi - r_lo + RT - 1) / RT;
                         my_dng += n_rt;
@@ -238,7 +242,7 @@ __global__ void __launch_bounds__(kPlanThreads, 1) plan_kernel(const AttnDev d, 
                       },
                       [&](int, const SegPlan& sp) {
                         my_dng += sp.n_rt;
-                        for (int rt = 0; rt < sp.n_rt; ++rt) my_tiles_g += kCausalFixedTiles + p.nt + seg_tiles(d, sp, rt, B);
+                        for (int rt = 0; rt < sp.n_rt; ++rt) my_tiles_g += kCausalFixedTiles + p.nt + seg_tiles(c, sp, rt, B);
                       });
     } else {
       my_sq += p.npc * p.n_rows;
@@ -249,11 +253,11 @@ __global__ void __launch_bounds__(kPlanThreads, 1) plan_kernel(const AttnDev d, 
   const int sper = (NS + kPlanThreads - 1) / kPlanThreads;
   const int s_lo = min(tid * sper, NS), s_hi = min(s_lo + sper, NS);
   for (int s = s_lo; s < s_hi; ++s) {
-    const SegPlan p = seg_plan(d, s, B);
-    if (seg_joined_group(d, p, B, dense_ok) >= 0) continue;  // counted with its group
+    const SegPlan p = seg_plan(c, s, B);
+    if (seg_joined_group(c, p, B, dense_ok) >= 0) continue;  // counted with its group
     if (dense_ok) {
       my_dns += p.n_rt;
-      for (int rt = 0; rt < p.n_rt; ++rt) my_tiles_s += kCausalFixedTiles + seg_tiles(d, p, rt, B);
+      for (int rt = 0; rt < p.n_rt; ++rt) my_tiles_s += kCausalFixedTiles + seg_tiles(c, p, rt, B);
     } else {
       for (int i = 0; i < p.n; ++i) {
         const int nb = (p.kv - p.n + i + 1 + B - 1) / B;
@@ -268,7 +272,7 @@ __global__ void __launch_bounds__(kPlanThreads, 1) plan_kernel(const AttnDev d, 
   const int o_lo = min(tid * oper, NO), o_hi = min(o_lo + oper, NO);
   int my_dno = 0, my_tiles_o = 0;
   for (int o = o_lo; o < o_hi; ++o) {
-    const GroupPlan p = outer_plan(d, o, B, dense_ok);
+    const GroupPlan p = outer_plan(c, o, B, dense_ok);
     if (p.dense) { my_dno += p.n_rt; my_tiles_o += p.n_rt * p.nt; }
     else { my_sq += p.npc * p.n_rows; my_blocks += (long long)p.nblk * p.n_rows; }
   }
@@ -297,11 +301,16 @@ __global__ void __launch_bounds__(kPlanThreads, 1) plan_kernel(const AttnDev d, 
   const int sqs_base = scan[5];
 
   const bool overflow = (total_dn > d.cap_dn) || (total_sq + total_sqs > d.cap_sq);
+  // From here on the workspace is written: the kernel before this one has to be complete (see count_hdr), and the
+  // attention kernels, which wait only for their direct predecessor, find it complete too.
+  pdl_wait();
   if (tid == 0) {
+    d.hdr[kHdrStatus] = max(count_hdr[kHdrStatus], overflow ? kStatusListOverflow : kStatusOk);
+    d.hdr[kHdrSqCounter] = 0;
+    d.hdr[kHdrPlannedSlots] = (d.slot_mapping && NS == 0 && !d.head_mapping) ? 1 : 0;
     d.hdr[kHdrNumSq] = overflow ? 0 : total_sq + total_sqs;
     d.hdr[kHdrNumDn] = overflow ? 0 : total_dn;
     d.hdr[kHdrDnTiles] = overflow ? 0 : total_tiles * d.num_heads;
-    if (overflow) atomicMax(&d.hdr[kHdrStatus], kStatusListOverflow);
     // Split of the SMs between the dense kernel and the single-query kernel that runs beside it:
     // proportional to their work in units of one 128-token kv tile of one head (64 KiB of KV for
     // the streaming kernel). A dense tile is weighted: giving the dense kernel too many SMs costs
@@ -318,7 +327,8 @@ __global__ void __launch_bounds__(kPlanThreads, 1) plan_kernel(const AttnDev d, 
     if (d.dense_ctas > 0) c = min(d.dense_ctas, sms);  // the caller's choice
     d.hdr[kHdrDenseCtas] = c;
   }
-  if (overflow) { pdl_wait(); return; }
+  if (overflow) return;
+  __syncthreads();  // the header's status is in place; faults found below are added to it
 
   // ---- groups: dense items (whole prefix per row tile) or single-query prefix items per row ----
   for (int g = g_lo; g < g_hi; ++g) {
@@ -536,10 +546,6 @@ __global__ void __launch_bounds__(kPlanThreads, 1) plan_kernel(const AttnDev d, 
       d.sq_items[total_sq + idx] = it;
     }
   }
-  // The planner reads nothing the kernel before it writes (a KV fill, which lets its dependents
-  // start early), so it runs beside that kernel; it still must not COMPLETE before it, because the
-  // attention kernels wait only for their direct predecessor, the planner.
-  pdl_wait();
 }
 
 }  // namespace

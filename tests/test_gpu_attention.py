@@ -764,3 +764,37 @@ def test_head_shards_equal_the_unsharded_result():
     rows = sample_rows(wl, 12, seed=3)
     ref = oracle_for_workload(wl, full, rows=rows)
     assert_close_to_oracle(joined[rows], ref, wl.dtype, "head shards joined")
+
+
+def test_calls_of_different_layouts_on_one_scratch():
+    """One-shot calls back to back on ONE workspace, none waiting for the one before on the host. Their lists
+    and partials lie at different offsets, so a planner that wrote its lists while the merge of the call
+    before still read its partials would change that call's result (prefill rows x 32 heads: a long merge)."""
+    wls = [make_workload(4, shrink=8, num_heads=32), make_workload(2, shrink=1, num_heads=32), make_workload(1, num_heads=4),
+           make_workload(3, shrink=8, num_heads=40)]
+    tensors = [wl.materialize(DEV) for wl in wls]
+
+    def call_of(wl, t, workspace=None):
+        return pb.AttentionCall(
+            num_rows=wl.num_rows, num_heads=t["query"].shape[1], head_size=wl.head_size, block_size=wl.block_size, dtype=wl.dtype,
+            device=t["query"].device, suffix_lens=t["suffix_lens"], suffix_tables=t["suffix_tables"],
+            group_row_offsets=t["group_row_offsets"], group_prefix_lens=t["group_prefix_lens"], group_tables=t["group_tables"],
+            seg_row_offsets=t.get("seg_row_offsets"), seg_kv_lens=t.get("seg_kv_lens"), seg_tables=t.get("seg_tables"),
+            workspace=workspace)
+
+    alone = []
+    for wl, t in zip(wls, tensors):
+        call = call_of(wl, t)
+        alone.append(call.run(t["query"], torch.empty_like(t["query"]), t["key_cache"], t["value_cache"]))
+        assert call.status() == 0
+    assert wls[0].num_rows >= 1024
+    shared = torch.empty(max(call_of(wl, t).workspace_bytes for wl, t in zip(wls, tensors)), dtype=torch.uint8, device=DEV)
+    calls = [call_of(wl, t, shared) for wl, t in zip(wls, tensors)]
+    order = np.random.default_rng(0).integers(0, len(wls), size=60).tolist() + [0, 1, 0, 3, 0, 2, 0]
+    outs = []
+    for i in order:
+        t = tensors[i]
+        outs.append(calls[i].run(t["query"], torch.empty_like(t["query"]), t["key_cache"], t["value_cache"]))
+    torch.cuda.synchronize()
+    for i, out in zip(order, outs):
+        assert torch.equal(out, alone[i])
