@@ -327,7 +327,12 @@ __global__ void __launch_bounds__(kPlanThreads, 1) plan_kernel(const AttnDev d, 
     if (d.dense_ctas > 0) c = min(d.dense_ctas, sms);  // the caller's choice
     d.hdr[kHdrDenseCtas] = c;
   }
-  if (overflow) return;
+  if (overflow) {  // no lists: no row has a partial (the merge reads the row infos and writes NaN)
+    RowInfo none = {};
+    none.group = none.dn = none.seg_dn = none.odn = -1;
+    for (int r = tid; r < S; r += kPlanThreads) d.row_info[r] = none;
+    return;
+  }
   __syncthreads();  // the header's status is in place; faults found below are added to it
 
   // ---- groups: dense items (whole prefix per row tile) or single-query prefix items per row ----

@@ -798,3 +798,20 @@ def test_calls_of_different_layouts_on_one_scratch():
     torch.cuda.synchronize()
     for i, out in zip(order, outs):
         assert torch.equal(out, alone[i])
+
+
+@pytest.mark.parametrize("dense_min_rows", [0, 1 << 30])
+def test_lists_that_do_not_fit_are_reported(dense_min_rows):
+    """Row offsets that run back and forth make every other group cover all rows: more items than the lists
+    hold. Nothing is planned, the status says so and the output is NaN, whatever the workspace held before."""
+    q, kc, vc, meta = _mini(torch.float16, 2, 64, [20] * 512, nb=1040, seed=7)
+    g = 64
+    i32 = lambda a: torch.tensor(a, dtype=torch.int32, device=DEV)
+    call = pb.AttentionCall(
+        num_rows=512, num_heads=2, head_size=128, block_size=16, dtype=q.dtype, device=q.device, suffix_lens=i32(meta["sl"]),
+        suffix_tables=i32(meta["st"]), group_row_offsets=i32([0, 512] * (g // 2) + [0]), group_prefix_lens=i32([64] * g),
+        group_tables=i32(meta["gt"] * g), dense_min_rows=dense_min_rows)
+    call.workspace.fill_(0x7F)
+    out = torch.zeros_like(q)
+    call.run(q, out, kc, vc)
+    assert call.status() == 3 and torch.isnan(out).all()
