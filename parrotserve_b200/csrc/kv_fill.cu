@@ -25,6 +25,17 @@ __device__ __forceinline__ long long load_slot(const void* slots, int is64, long
               : (long long)reinterpret_cast<const int*>(slots)[t];
 }
 
+// Kernels launched with programmatic serialization begin while the kernel before them still writes: what
+// they read (rows, cache cells, cos/sin) is only settled after pdl_wait(). Their loads must therefore be
+// ordinary ones; the read-only path (__ldg, or const __restrict__ parameters, which the compiler may turn into
+// it) asks for data that nobody writes during the whole life of the kernel. Hence no __restrict__ in those
+// kernels, and loads that are to be in flight together are written as load16() into registers first.
+__device__ __forceinline__ uint4 load16(const void* p) {
+  uint4 v;
+  asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
+
 template <int E> struct ElemOf;
 template <> struct ElemOf<2> { using type = uint16_t; };
 template <> struct ElemOf<4> { using type = uint32_t; };
@@ -46,11 +57,11 @@ __device__ __forceinline__ int run_length(unsigned cont, int lane_of_first) {
 // FILL == true : scatter rows into the cache.   FILL == false : gather rows out of the cache.
 template <int E, bool FILL>
 __global__ void __launch_bounds__(kFillWarps * 32) kv_run_kernel(
-    uint8_t* __restrict__ key, uint8_t* __restrict__ value, uint8_t* __restrict__ kcache,
-    uint8_t* __restrict__ vcache, const void* __restrict__ slots, const int is64,
+    uint8_t* key, uint8_t* value, uint8_t* kcache,
+    uint8_t* vcache, const void* slots, const int is64,
     const long long T, const int H, const int D, const int B, const long long key_stride,
     const long long value_stride, const long long kbs, const long long khs,
-    const long long num_blocks, int* __restrict__ status) {
+    const long long num_blocks, int* status) {
   using elem_t = typename ElemOf<E>::type;
   extern __shared__ __align__(16) uint8_t smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -99,7 +110,7 @@ __global__ void __launch_bounds__(kFillWarps * 32) kv_run_kernel(
           const int i = idx / nch, c = idx - i * nch;
           const uint4* row = reinterpret_cast<const uint4*>(key + ((size_t)(t + i) * key_stride + (size_t)h * D) * E) + c;
           const uint4* cell = reinterpret_cast<const uint4*>(kt) + (size_t)c * B + off0 + i;
-          tmp[u] = FILL ? *row : *cell;
+          tmp[u] = load16(FILL ? row : cell);
         }
       }
 #pragma unroll
@@ -122,7 +133,7 @@ __global__ void __launch_bounds__(kFillWarps * 32) kv_run_kernel(
           const int idx = base + u * 32 + lane;
           if (idx < run * nch) {
             const int i = idx / nch, c = idx - i * nch;
-            tmp[u] = *(reinterpret_cast<const uint4*>(value + ((size_t)(t + i) * value_stride + (size_t)h * D) * E) + c);
+            tmp[u] = load16(value + ((size_t)(t + i) * value_stride + (size_t)h * D + c * kVec) * E);
           }
         }
 #pragma unroll
@@ -205,8 +216,8 @@ __device__ __forceinline__ void rotate_pair(const uint4& x, const uint4& y, cons
   float fx[kVec], fy[kVec], fc[kVec], fs[kVec], rx[kVec], ry[kVec];
   unpack16<T>(x, fx);
   unpack16<T>(y, fy);
-  unpack16<T>(reinterpret_cast<const uint4*>(cs)[cx], fc);
-  unpack16<T>(reinterpret_cast<const uint4*>(cs)[half_chunks + cx], fs);
+  unpack16<T>(load16(cs + cx * 16), fc);
+  unpack16<T>(load16(cs + (half_chunks + cx) * 16), fs);
 #pragma unroll
   for (int j = 0; j < kVec; ++j) {
     rx[j] = fx[j] * fc[j] - fy[j] * fs[j];
@@ -218,9 +229,9 @@ __device__ __forceinline__ void rotate_pair(const uint4& x, const uint4& y, cons
 
 template <typename T>
 __global__ void __launch_bounds__(kFillWarps * 32) rotary_fill_kernel(
-    uint8_t* __restrict__ query, uint8_t* __restrict__ key, const uint8_t* __restrict__ value,
-    uint8_t* __restrict__ kcache, uint8_t* __restrict__ vcache, const void* __restrict__ slots, const int is64,
-    const long long* __restrict__ positions, const uint8_t* __restrict__ cos_sin, const int rot_dim,
+    uint8_t* query, uint8_t* key, const uint8_t* value,
+    uint8_t* kcache, uint8_t* vcache, const void* slots, const int is64,
+    const long long* positions, const uint8_t* cos_sin, const int rot_dim,
     const long long max_pos, const long long T_tok, const int Hq, const int H, const int D, const int B,
     const long long q_stride, const long long key_stride, const long long value_stride, const long long kbs,
     const long long khs, const long long num_blocks, const int write_key_back) {
@@ -248,7 +259,7 @@ __global__ void __launch_bounds__(kFillWarps * 32) rotary_fill_kernel(
       uint4* row = reinterpret_cast<uint4*>(query + ((size_t)t * q_stride + (size_t)h * D) * E);
       for (int u = lane; u < half; u += 32) {
         uint4 ox, oy;
-        rotate_pair<T>(row[u], row[u + half], cs, u, half, ox, oy);
+        rotate_pair<T>(load16(row + u), load16(row + u + half), cs, u, half, ox, oy);
         row[u] = ox;
         row[u + half] = oy;
       }
@@ -262,7 +273,7 @@ __global__ void __launch_bounds__(kFillWarps * 32) rotary_fill_kernel(
       uint4* row = reinterpret_cast<uint4*>(key + ((size_t)t * key_stride + (size_t)h * D) * E);
       for (int u = lane; u < half; u += 32) {
         uint4 ox, oy;
-        rotate_pair<T>(row[u], row[u + half], cs, u, half, ox, oy);
+        rotate_pair<T>(load16(row + u), load16(row + u + half), cs, u, half, ox, oy);
         row[u] = ox;
         row[u + half] = oy;
       }
@@ -297,20 +308,19 @@ __global__ void __launch_bounds__(kFillWarps * 32) rotary_fill_kernel(
       uint4* cell = reinterpret_cast<uint4*>(kt) + off0 + i;
       if (u < half) {
         uint4 ox, oy;
-        rotate_pair<T>(row[u], row[u + half], cs_row(t + i), u, half, ox, oy);
+        rotate_pair<T>(load16(row + u), load16(row + u + half), cs_row(t + i), u, half, ox, oy);
         cell[(size_t)u * B] = ox;
         cell[(size_t)(u + half) * B] = oy;
         if (write_key_back) { row[u] = ox; row[u + half] = oy; }
       } else {
         const int c = u + half;
-        cell[(size_t)c * B] = row[c];
+        cell[(size_t)c * B] = load16(row + c);
       }
     }
     // V: transposed through shared memory, full blocks written with 16-byte stores
     for (int idx = lane; idx < run * nch; idx += 32) {
       const int i = idx / nch, c = idx - i * nch;
-      const uint4* row = reinterpret_cast<const uint4*>(value + ((size_t)(t + i) * value_stride + (size_t)h * D) * E) + c;
-      reinterpret_cast<uint4*>(tile)[i * nch + c] = *row;
+      reinterpret_cast<uint4*>(tile)[i * nch + c] = load16(value + ((size_t)(t + i) * value_stride + (size_t)h * D + c * kVec) * E);
     }
     __syncwarp();
     const elem_t* ts = reinterpret_cast<const elem_t*>(tile);
@@ -350,9 +360,9 @@ constexpr int win_heads(bool rot) { return rot ? 4 : 2; }
 
 template <typename T, bool ROT>
 __global__ void __launch_bounds__(128) fill_window_kernel(
-    uint8_t* __restrict__ query, uint8_t* __restrict__ key, const uint8_t* __restrict__ value,
-    uint8_t* __restrict__ kcache, uint8_t* __restrict__ vcache, const void* __restrict__ slots, const int is64,
-    const long long* __restrict__ positions, const uint8_t* __restrict__ cos_sin, const int rot_dim,
+    uint8_t* query, uint8_t* key, const uint8_t* value,
+    uint8_t* kcache, uint8_t* vcache, const void* slots, const int is64,
+    const long long* positions, const uint8_t* cos_sin, const int rot_dim,
     const long long max_pos, const long long T_tok, const int Hq, const int H, const int D,
     const long long q_stride, const long long key_stride, const long long value_stride, const long long kbs,
     const long long khs, const long long num_blocks, const int write_key_back) {
@@ -381,13 +391,13 @@ __global__ void __launch_bounds__(128) fill_window_kernel(
     for (int k = 0; k < kWinHeads; ++k) {
       if (h0 + k < heads) {
         const uint4* row = reinterpret_cast<const uint4*>(row0 + (size_t)(h0 + k) * D * E);
-        x[k] = row[u];
-        y[k] = row[u + half];
+        x[k] = load16(row + u);
+        y[k] = load16(row + u + half);
       }
     }
     float fc[kVec], fs[kVec];
-    unpack16<T>(__ldg(reinterpret_cast<const uint4*>(cs) + u), fc);
-    unpack16<T>(__ldg(reinterpret_cast<const uint4*>(cs) + half + u), fs);
+    unpack16<T>(load16(cs + u * 16), fc);
+    unpack16<T>(load16(cs + (half + u) * 16), fs);
 #pragma unroll
     for (int k = 0; k < kWinHeads; ++k) {
       if (h0 + k < heads) {
@@ -459,7 +469,7 @@ __global__ void __launch_bounds__(128) fill_window_kernel(
       uint4 v[kWinHeads];
 #pragma unroll
       for (int k = 0; k < kWinHeads; ++k)
-        if (h0 + k < H) v[k] = reinterpret_cast<const uint4*>(krow + (size_t)(h0 + k) * D * E)[c];
+        if (h0 + k < H) v[k] = load16(krow + (size_t)(h0 + k) * D * E + c * 16);
 #pragma unroll
       for (int k = 0; k < kWinHeads; ++k)
         if (h0 + k < H) cell(h0 + k)[(size_t)c * B] = v[k];
@@ -488,8 +498,8 @@ __global__ void __launch_bounds__(128) fill_window_kernel(
         for (int k = 0; k < kWinHeads; ++k) {
           if (h0 + k < H) {
             const uint8_t* p = rows + (size_t)(h0 + k) * D * E + c * 16;
-            a[k] = __ldg(reinterpret_cast<const uint4*>(p));
-            b[k] = __ldg(reinterpret_cast<const uint4*>(p + next));
+            a[k] = load16(p);
+            b[k] = load16(p + next);
           }
         }
 #pragma unroll
@@ -522,7 +532,7 @@ __global__ void __launch_bounds__(128) fill_window_kernel(
       uint4 v[kWinHeads];
 #pragma unroll
       for (int k = 0; k < kWinHeads; ++k)
-        if (h0 + k < H) v[k] = __ldg(reinterpret_cast<const uint4*>(row + (size_t)(h0 + k) * D * E) + c);
+        if (h0 + k < H) v[k] = load16(row + (size_t)(h0 + k) * D * E + c * 16);
 #pragma unroll
       for (int k = 0; k < kWinHeads; ++k) {
         if (h0 + k < H) {
@@ -544,10 +554,10 @@ __global__ void __launch_bounds__(128) fill_window_kernel(
 // K and V of 8090 tokens x 32 heads x 128 (fp16, 265 MB read and written): 127 -> 57 us, 4.6 TB/s.
 template <int E, bool IS_V>
 __global__ void __launch_bounds__(128) move_runs_kernel(
-    const uint8_t* __restrict__ cache, uint8_t* __restrict__ dest, const long long* __restrict__ src_slots,
-    const long long* __restrict__ dest_idx, const long long n, const int H, const int heads_per_cta, const int D,
+    const uint8_t* cache, uint8_t* dest, const long long* src_slots,
+    const long long* dest_idx, const long long n, const int H, const int heads_per_cta, const int D,
     const long long dest_stride, const long long kbs, const long long khs, const long long num_blocks,
-    const long long dest_rows, int* __restrict__ status) {
+    const long long dest_rows, int* status) {
   constexpr int B = 16;
   constexpr int kVec = 16 / E;
   extern __shared__ __align__(16) uint8_t smem[];
@@ -584,8 +594,8 @@ __global__ void __launch_bounds__(128) move_runs_kernel(
         if (half * 8 < off + run && half * 8 + 8 > off) {
 #pragma unroll 4
           for (int p = lane >> 1; p < D / 2; p += 16) {
-            const uint4 a = __ldg(reinterpret_cast<const uint4*>(src + (size_t)p * 64 + half * 16));
-            const uint4 b = __ldg(reinterpret_cast<const uint4*>(src + (size_t)p * 64 + 32 + half * 16));
+            const uint4 a = load16(src + (size_t)p * 64 + half * 16);
+            const uint4 b = load16(src + (size_t)p * 64 + 32 + half * 16);
             const uint32_t av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
@@ -599,7 +609,7 @@ __global__ void __launch_bounds__(128) move_runs_kernel(
         if (quarter * 4 < off + run && quarter * 4 + 4 > off) {
 #pragma unroll 4
           for (int d = lane >> 2; d < D; d += 8) {
-            const uint4 a = __ldg(reinterpret_cast<const uint4*>(src + (size_t)d * 64 + quarter * 16));
+            const uint4 a = load16(src + (size_t)d * 64 + quarter * 16);
             tile[(quarter * 4 + 0) * pitch + d] = a.x;
             tile[(quarter * 4 + 1) * pitch + d] = a.y;
             tile[(quarter * 4 + 2) * pitch + d] = a.z;
@@ -623,8 +633,15 @@ __global__ void __launch_bounds__(128) move_runs_kernel(
       const uint4* cell = reinterpret_cast<const uint4*>(src) + off + i;
       uint4* row = reinterpret_cast<uint4*>(dest + ((size_t)(live ? to : 0) * dest_stride + (size_t)h * D) * E);
       if (live) {
-#pragma unroll 8
-        for (int c = lane & 1; c < nch; c += 2) row[c] = __ldg(cell + (size_t)c * B);
+        for (int base = lane & 1; base < nch; base += 16) {
+          uint4 v[8];
+#pragma unroll
+          for (int u = 0; u < 8; ++u)
+            if (base + 2 * u < nch) v[u] = load16(cell + (size_t)(base + 2 * u) * B);
+#pragma unroll
+          for (int u = 0; u < 8; ++u)
+            if (base + 2 * u < nch) row[base + 2 * u] = v[u];
+        }
       }
       __syncwarp();
     }

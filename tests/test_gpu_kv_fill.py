@@ -266,3 +266,33 @@ def test_copy_blocks_and_swap_blocks_bit_exact(dtype):
         assert np.array_equal(bits(kcs[1][dd]), bits(host[s]))
     with pytest.raises(RuntimeError):  # a block outside the destination cache is refused before anything is copied
         cache_ops.swap_blocks(kcs[0], host, {0: 24})
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+@pytest.mark.parametrize("scattered", [False, True])
+def test_moves_right_behind_fills_see_the_new_rows(dtype, scattered):
+    """The kernels of a fill and of a move are launched while the one before still runs. Fills of the same
+    slots with other rows each time, every one followed at once by both moves out of the cache and by a fill of
+    a second cache from the moved rows: each reads what the one before has just written, bit for bit."""
+    h, d, b, nb, t, rounds = 8, 128, 16, 200, 2050, 24
+    kc, vc, g = _caches(dtype, nb, h, d, b, 3)
+    k2, v2 = torch.zeros_like(kc), torch.zeros_like(vc)
+    rng = np.random.default_rng(4)
+    blocks = rng.permutation(nb)
+    slots = rng.permutation(nb * b)[:t] if scattered else (blocks[:, None] * b + np.arange(b)).reshape(-1)[:t]
+    slots = torch.tensor(slots, device=DEV)
+    dst = torch.arange(t, device=DEV)
+    keys = [torch.randn((t, h, d), generator=g, device=DEV).to(dtype) for _ in range(rounds)]
+    values = [torch.randn((t, h, d), generator=g, device=DEV).to(dtype) for _ in range(rounds)]
+    rows = [(torch.empty_like(k), torch.empty_like(k), torch.empty_like(k), torch.empty_like(k)) for k in keys]
+    torch.cuda.synchronize()
+    for k, v, (ko, vo, kb, vb) in zip(keys, values, rows):
+        pb.vllm_reshape_and_cache(k, v, kc, vc, slots)
+        pb.move_tokens_from_blocked_v_cache(vc, vo, slots, dst)
+        pb.move_tokens_from_blocked_k_cache(kc, ko, slots, dst)
+        pb.vllm_reshape_and_cache(ko, vo, k2, v2, slots)
+        pb.move_tokens_from_blocked_k_cache(k2, kb, slots, dst)
+        pb.move_tokens_from_blocked_v_cache(v2, vb, slots, dst)
+    torch.cuda.synchronize()
+    for k, v, (ko, vo, kb, vb) in zip(keys, values, rows):
+        assert torch.equal(ko, k) and torch.equal(vo, v) and torch.equal(kb, k) and torch.equal(vb, v)
