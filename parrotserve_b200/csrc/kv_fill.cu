@@ -5,10 +5,11 @@
 //   move   : dest[dest_idx[i]] = row of slot src_slots[i] (K or V)
 //   rows   : dest[dest_idx[i]] = src[src_idx[i]] over plain rows
 //
-// A run of tokens whose slots are consecutive inside one physical block (prefill) is handled
-// by one warp per head: K moves as 16-byte chunks, V is transposed through shared memory so a
-// full block is written with 16-byte stores; a lone decode token degenerates to the scattered
-// element writes the layout forces.
+// Runs of tokens whose slots are consecutive inside one physical block (prefill) share sectors of the V tiles and
+// are written together; a lone decode token degenerates to the scattered element writes the layout forces.
+// Block size 16 (the engine's): fills, rotary and moves take windows of 16 tokens (fill_window_kernel,
+// move_runs_kernel). Other block sizes, and every gather, take a warp per (run, head): K as 16-byte chunks, V
+// transposed through shared memory so that a full block is written with 16-byte stores (kv_run_kernel).
 //
 // Reference counterparts: reshape_and_cache_kernel / gather_cached_kv_kernel
 // (3rdparty/vllm/csrc/cache_kernels.cu:142-182, 229-344) and the Triton movers
@@ -39,6 +40,17 @@ __device__ __forceinline__ uint4 load16(const void* p) {
 template <int E> struct ElemOf;
 template <> struct ElemOf<2> { using type = uint16_t; };
 template <> struct ElemOf<4> { using type = uint32_t; };
+template <typename T> __device__ __forceinline__ T load_elem(const void* p);
+template <> __device__ __forceinline__ uint16_t load_elem<uint16_t>(const void* p) {
+  uint16_t v;
+  asm volatile("ld.global.u16 %0, [%1];" : "=h"(v) : "l"(p));
+  return v;
+}
+template <> __device__ __forceinline__ uint32_t load_elem<uint32_t>(const void* p) {
+  uint32_t v;
+  asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p));
+  return v;
+}
 
 // Runs of a list of slots: lane l of the warp holds entry first - 1 + l (its slot, or a negative number
 // outside the list). A run is a maximal stretch of entries with consecutive slots inside one block of 16;
@@ -345,20 +357,43 @@ __global__ void __launch_bounds__(kFillWarps * 32) rotary_fill_kernel(
 // tokens and kWinHeads heads; every thread owns one (token, chunk) and walks the heads, so that the loads of
 // all of them are in flight together and the cos/sin values are read once for them. q and k need no more
 // than the token's own slot: neighbouring lanes are neighbouring tokens, whose cells of a block are
-// neighbours too. V goes from rows to tiles [d][16 tokens]: two tokens of a run share a 4-byte word, so a
-// thread reads the same chunk of both, and eight lanes write one whole 32-byte row of the tile; nothing goes
-// through shared memory. The runs that START among the CTA's tokens are written by it up to their end, so
-// that a full block's sectors are written whole; a window with more than kFewRuns of them (decode tokens) is
-// written token by token. What bounds it is memory. 10 842 tokens (16
-// prefills, 240 decodes) x 32 heads, fp16: rotary and fill 165 -> 118 us (4.5 TB/s of 534 MB) against a CTA per
-// token of which fifteen of sixteen left at once; the plain fill of 8767 prefill tokens about 65 -> 52 us.
-// Heads per CTA: rotary 2: 125 us, 4: 118; plain fill 4: 430 us with the attention behind it, 2: 426. At most 96
-// registers (five CTAs an SM): 129 us; q in CTAs of its own: 130 us.
-constexpr int kFewRuns = 2;
+// neighbours too. V goes from rows to tiles [d][16 tokens]. The runs of consecutive slots that START among the
+// CTA's tokens are written by it up to their end, so that a full block's sectors are written whole. Two forms:
+//   long runs (prefill): two tokens of a run share a 4-byte word, so a thread reads the same chunk of both, and
+//     eight lanes write one whole 32-byte row of the tile; nothing goes through shared memory. (fp32: a thread per
+//     token and chunk; eight lanes are 32 bytes of a tile row.)
+//   short ones (decode tokens): a warp per (token, head) with its lanes along d. Every element is a sector of its
+//     own then, and the lanes of a store fall into eight 128-byte lines. (With a thread per token and chunk they fall
+//     into 32, and the store unit of an SM takes a line at a time: 1024 lone tokens x 32 heads, fp16, 83 us against 49;
+//     with the warp per run of the other block sizes 49.)
+// Which form: by the mean length of a window's runs. Runs of five, 2000 tokens x 32 heads: fp16 37 us by runs, 53
+// by elements, fp32 55 and 87; runs of three: fp16 76 and 73, fp32 85 and 114.
+// What bounds it is memory. 10 842 tokens (16 prefills, 240 decodes) x 32 heads, fp16: rotary and fill
+// 165 -> 114 us (4.7 TB/s of 534 MB) against a CTA per token of which fifteen of sixteen left at once; the plain
+// fill of 8767 prefill tokens about 65 -> 52 us.
+constexpr int kMeanRun16 = 4, kMeanRun32 = 3;  // by runs from this mean length on: 16-bit types, fp32
 
-constexpr int win_heads(bool rot) { return rot ? 4 : 2; }
+// Heads per CTA: one in small batches, so that the stores spread over the chip (1024 lone tokens x 32 heads 53 us with
+// two heads, 49 with one); then 4 with rotation (2: 125 us for the 10 842 tokens above, 4: 118) and 2 without (4: 430 us
+// with the attention behind it, 2: 426). Small is, in (window, head) pairs per SM: 16 without rotation (8192 tokens x 32
+// heads in whole blocks, 111 per SM: 49 us with two, 57 with one; 2048 x 8, 7 per SM: the same) and 6 with it, where
+// the heads share cos and sin (2048 tokens x 8 heads in whole blocks, 7 per SM: 6.8 us with four, 8.0 with one; 256 lone
+// tokens x 32 heads, 3.5 per SM: 15.2 and 10.8).
+constexpr int win_heads(bool rot, bool small) { return small ? 1 : rot ? 4 : 2; }
+// The smallest batches have CTAs of their own for (q,) K and V, whose trips to memory then run beside each other, as
+// long as every CTA finds an SM to itself: 64 lone tokens x 8 heads with rotation 4.8 us together, 3.7 apart; with 32
+// heads, two CTAs an SM, the plain fill takes 4.5 together and 5.5 apart.
+struct WinShape {
+  bool small;
+  unsigned roles;
+};
+static WinShape win_shape(long long tokens, int heads, bool rot) {
+  const long long pairs = (tokens + 15) / 16 * heads;
+  const int sms = sm_count(), roles = rot ? 3 : 2;
+  return WinShape{pairs <= (rot ? 6 : 16) * sms, pairs * roles <= sms ? (unsigned)roles : 1u};
+}
 
-template <typename T, bool ROT>
+template <typename T, bool ROT, bool SMALL>
 __global__ void __launch_bounds__(128) fill_window_kernel(
     uint8_t* query, uint8_t* key, const uint8_t* value,
     uint8_t* kcache, uint8_t* vcache, const void* slots, const int is64,
@@ -367,12 +402,15 @@ __global__ void __launch_bounds__(128) fill_window_kernel(
     const long long q_stride, const long long key_stride, const long long value_stride, const long long kbs,
     const long long khs, const long long num_blocks, const int write_key_back) {
   constexpr int B = 16;
-  constexpr int kWinHeads = win_heads(ROT);
+  constexpr int kWinHeads = win_heads(ROT, SMALL);
   constexpr int E = (int)sizeof(T);
   constexpr int kVec = 16 / E;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const long long first = (long long)blockIdx.x * 16;
   const int h0 = blockIdx.y * kWinHeads;
+  // the smallest batches have CTAs of their own for q, K and V (blockIdx.z)
+  const bool all = !SMALL || gridDim.z == 1;
+  const bool do_q = ROT && (all || blockIdx.z == 0), do_k = all || blockIdx.z == (ROT ? 1 : 0), do_v = all || blockIdx.z == (ROT ? 2 : 1);
   // resident while the kernel before this one drains: wait for it before reading anything, then let the
   // next kernel set itself up (it waits before it reads the cache)
   pdl_wait();
@@ -414,7 +452,7 @@ __global__ void __launch_bounds__(128) fill_window_kernel(
     }
   };
 
-  if (ROT) {  // q in place; with no cache k too (eight lanes: 128 contiguous bytes of a row)
+  if (do_q) {  // q in place; with no cache k too (eight lanes: 128 contiguous bytes of a row)
     const long long tok = first + warp * 4 + (lane >> 3);
     if (tok < T_tok) {
       const uint8_t* cs = cs_row(tok);
@@ -435,9 +473,8 @@ __global__ void __launch_bounds__(128) fill_window_kernel(
         }
       }
     }
-    if (kcache == nullptr) return;
   }
-  if (h0 >= H) return;
+  if (h0 >= H || kcache == nullptr || !(do_k || do_v)) return;
 
   // lane l: the slot of token first - 1 + l (negative: none, or outside the cache)
   const long long my = first - 1 + lane;
@@ -447,7 +484,7 @@ __global__ void __launch_bounds__(128) fill_window_kernel(
   // ---- K: token `i` of the window, chunks g, g + 8, ... ----
   const int i = (lane & 7) + 8 * (warp & 1), g = (lane >> 3) + 4 * (warp >> 1);
   const long long s_i = __shfl_sync(0xffffffffu, slot, i + 1);
-  if (s_i >= 0) {
+  if (do_k && s_i >= 0) {
     uint8_t* krow = key + (size_t)(first + i) * key_stride * E;
     uint4* cell0 = reinterpret_cast<uint4*>(kcache + (size_t)(s_i / B) * kbs * E) + (s_i & (B - 1));
     auto cell = [&](int h) { return reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(cell0) + (size_t)h * khs * E); };
@@ -464,23 +501,30 @@ __global__ void __launch_bounds__(128) fill_window_kernel(
           }
         });
     }
-#pragma unroll 2
-    for (int c = 2 * half + g; c < nch; c += 8) {
-      uint4 v[kWinHeads];
+    constexpr int kChunks = SMALL ? 4 : 2;  // chunks per head in flight
+    for (int c0 = 2 * half + g; c0 < nch; c0 += 8 * kChunks) {
+      uint4 v[kChunks][kWinHeads];
 #pragma unroll
-      for (int k = 0; k < kWinHeads; ++k)
-        if (h0 + k < H) v[k] = load16(krow + (size_t)(h0 + k) * D * E + c * 16);
+      for (int u = 0; u < kChunks; ++u)
 #pragma unroll
-      for (int k = 0; k < kWinHeads; ++k)
-        if (h0 + k < H) cell(h0 + k)[(size_t)c * B] = v[k];
+        for (int k = 0; k < kWinHeads; ++k)
+          if (c0 + 8 * u < nch && h0 + k < H) v[u][k] = load16(krow + (size_t)(h0 + k) * D * E + (c0 + 8 * u) * 16);
+#pragma unroll
+      for (int u = 0; u < kChunks; ++u)
+#pragma unroll
+        for (int k = 0; k < kWinHeads; ++k)
+          if (c0 + 8 * u < nch && h0 + k < H) cell(h0 + k)[(size_t)(c0 + 8 * u) * B] = v[u][k];
     }
   }
 
   // ---- V: the runs that start among tokens first .. first + 15 (lanes 1 .. 16) ----
   const unsigned cont = run_continues(slot);
   const unsigned starts = ~cont & __ballot_sync(0xffffffffu, slot >= 0) & 0x1fffeu;
-  if (starts == 0) return;
-  if (E == 2 && __popc(starts) <= kFewRuns) {
+  if (starts == 0 || !do_v) return;
+  // lanes [lo, hi) hold the tokens of those runs
+  const int last = 31 - __clz(starts), lo = __ffs(starts) - 1, hi = last + run_length(cont, last);
+  const bool by_runs = hi - lo >= (E == 2 ? kMeanRun16 : kMeanRun32) * __popc(starts);
+  if (E == 2 && by_runs) {
     for (unsigned left = starts; left; left &= left - 1) {
       const int at = __ffs(left) - 1, run = run_length(cont, at);
       const long long s0 = __shfl_sync(0xffffffffu, slot, at);
@@ -519,29 +563,58 @@ __global__ void __launch_bounds__(128) fill_window_kernel(
     }
     return;
   }
-  // token by token: lanes [lo, hi) are the tokens of those runs
-  const int last = 31 - __clz(starts), lo = __ffs(starts) - 1, hi = last + run_length(cont, last);
   using elem_t = typename ElemOf<E>::type;
-  for (int base = lo; base < hi; base += 16) {
-    const int l = base + i;
-    const long long s = __shfl_sync(0xffffffffu, slot, min(l, 31));
-    if (l >= hi || s < 0) continue;
-    const uint8_t* row = value + (size_t)(first - 1 + l) * value_stride * E;
-    uint8_t* tile = vcache + ((size_t)(s / B) * kbs + (size_t)h0 * khs) * E + (s & (B - 1)) * E;
-    for (int c = g; c < nch; c += 8) {
-      uint4 v[kWinHeads];
+  if (E == 4 && by_runs) {  // eight lanes are eight tokens: 32 contiguous bytes of a tile row
+    for (int base = lo; base < hi; base += 16) {
+      const int l = base + i;
+      const long long s = __shfl_sync(0xffffffffu, slot, min(l, 31));
+      if (l >= hi || s < 0) continue;
+      const uint8_t* row = value + (size_t)(first - 1 + l) * value_stride * E;
+      uint8_t* tile = vcache + ((size_t)(s / B) * kbs + (size_t)h0 * khs) * E + (s & (B - 1)) * E;
+      for (int c = g; c < nch; c += 8) {
+        uint4 v[kWinHeads];
 #pragma unroll
-      for (int k = 0; k < kWinHeads; ++k)
-        if (h0 + k < H) v[k] = load16(row + (size_t)(h0 + k) * D * E + c * 16);
+        for (int k = 0; k < kWinHeads; ++k)
+          if (h0 + k < H) v[k] = load16(row + (size_t)(h0 + k) * D * E + c * 16);
 #pragma unroll
-      for (int k = 0; k < kWinHeads; ++k) {
-        if (h0 + k < H) {
-          const elem_t* e = reinterpret_cast<const elem_t*>(&v[k]);
-          uint8_t* out = tile + (size_t)k * khs * E + (size_t)c * 16 * B;
+        for (int k = 0; k < kWinHeads; ++k) {
+          if (h0 + k < H) {
+            const elem_t* e = reinterpret_cast<const elem_t*>(&v[k]);
+            uint8_t* out = tile + (size_t)k * khs * E + (size_t)c * 16 * B;
 #pragma unroll
-          for (int j = 0; j < kVec; ++j) *reinterpret_cast<elem_t*>(out + j * B * E) = e[j];
+            for (int j = 0; j < kVec; ++j) *reinterpret_cast<elem_t*>(out + j * B * E) = e[j];
+          }
         }
       }
+    }
+    return;
+  }
+  // a warp per (token, head), four of them at a time: all their loads in flight
+  constexpr int kBatch = 4, kSteps = 4;  // kSteps x 32 elements of a row
+  const int n_pairs = (hi - lo) * kWinHeads;
+  for (int p0 = warp; p0 < n_pairs; p0 += 4 * kBatch) {
+    const uint8_t* row[kBatch];
+    uint8_t* tile[kBatch];
+#pragma unroll
+    for (int u = 0; u < kBatch; ++u) {
+      const int p = min(p0 + 4 * u, n_pairs - 1);
+      const int l = lo + p / kWinHeads, h = h0 + p % kWinHeads;
+      const long long s = __shfl_sync(0xffffffffu, slot, l);
+      row[u] = (p0 + 4 * u < n_pairs && s >= 0 && h < H) ? value + ((size_t)(first - 1 + l) * value_stride + (size_t)h * D) * E : nullptr;
+      tile[u] = vcache + ((size_t)(s / B) * kbs + (size_t)h * khs + (s & (B - 1))) * E;
+    }
+    for (int d0 = lane; d0 < D; d0 += kSteps * 32) {
+      elem_t e[kBatch][kSteps];
+#pragma unroll
+      for (int u = 0; u < kBatch; ++u)
+#pragma unroll
+        for (int r = 0; r < kSteps; ++r)
+          if (row[u] && d0 + r * 32 < D) e[u][r] = load_elem<elem_t>(row[u] + (d0 + r * 32) * E);
+#pragma unroll
+      for (int u = 0; u < kBatch; ++u)
+#pragma unroll
+        for (int r = 0; r < kSteps; ++r)
+          if (row[u] && d0 + r * 32 < D) *reinterpret_cast<elem_t*>(tile[u] + (size_t)(d0 + r * 32) * B * E) = e[u][r];
     }
   }
 }
@@ -734,16 +807,18 @@ static int kv_run_launch(bool fill, void* key, void* value, void* kcache, void* 
   if (ks % vec || vs % vec || kbs % vec || khs % vec) return PB_ERR_INVALID_ARG;
   if (T > 0x7fffffffll) return PB_ERR_INVALID_ARG;
   if (fill && B == 16) {  // the engine's block size; the others take the warp per (run, head) below
-    const dim3 grid((unsigned)((T + 15) / 16), (unsigned)((H + win_heads(false) - 1) / win_heads(false)));
+    const WinShape shape = win_shape(T, H, false);
+    const bool small = shape.small;
+    const int per = win_heads(false, small);
+    const dim3 grid((unsigned)((T + 15) / 16), (unsigned)((H + per - 1) / per), shape.roles);
     const long long* no_pos = nullptr;
     const uint8_t* no_table = nullptr;
-    const cudaError_t err =
-        E == 2 ? launch_kernel(fill_window_kernel<__half, false>, grid, dim3(128), 0, s, true, (uint8_t*)nullptr, (uint8_t*)key,
-                               (const uint8_t*)value, (uint8_t*)kcache, (uint8_t*)vcache, slots, is64, no_pos, no_table, 0, 0ll,
-                               T, 0, H, D, 0ll, ks, vs, kbs, khs, num_blocks, 0)
-               : launch_kernel(fill_window_kernel<float, false>, grid, dim3(128), 0, s, true, (uint8_t*)nullptr, (uint8_t*)key,
-                               (const uint8_t*)value, (uint8_t*)kcache, (uint8_t*)vcache, slots, is64, no_pos, no_table, 0, 0ll,
-                               T, 0, H, D, 0ll, ks, vs, kbs, khs, num_blocks, 0);
+    auto launch = [&](auto kfn) {
+      return launch_kernel(kfn, grid, dim3(128), 0, s, true, (uint8_t*)nullptr, (uint8_t*)key, (const uint8_t*)value, (uint8_t*)kcache,
+                           (uint8_t*)vcache, slots, is64, no_pos, no_table, 0, 0ll, T, 0, H, D, 0ll, ks, vs, kbs, khs, num_blocks, 0);
+    };
+    const cudaError_t err = E == 2 ? (small ? launch(fill_window_kernel<__half, false, true>) : launch(fill_window_kernel<__half, false, false>))
+                                   : (small ? launch(fill_window_kernel<float, false, true>) : launch(fill_window_kernel<float, false, false>));
     if (err != cudaSuccess) { set_cuda_error(err); return PB_ERR_LAUNCH; }
     return PB_OK;
   }
@@ -776,10 +851,15 @@ static cudaError_t rotary_fill_launch_t(void* q, void* k, const void* v, void* k
                                         long long vs, long long kbs, long long khs, long long num_blocks, int write_back,
                                         cudaStream_t s) {
   if (B == 16) {  // the engine's block size (and rotation without a cache)
-    const dim3 win((unsigned)((T_tok + 15) / 16), (unsigned)(((Hq > H ? Hq : H) + win_heads(true) - 1) / win_heads(true)));
-    return launch_kernel(fill_window_kernel<T, true>, win, dim3(128), 0, s, true, (uint8_t*)q, (uint8_t*)k, (const uint8_t*)v,
-                         (uint8_t*)kc, (uint8_t*)vc, slots, is64, (const long long*)positions, (const uint8_t*)cos_sin, rot_dim,
-                         max_pos, T_tok, Hq, H, D, qs, ks, vs, kbs, khs, num_blocks, write_back);
+    const int heads = Hq > H ? Hq : H;
+    const WinShape shape = win_shape(T_tok, heads, true);
+    const bool small = shape.small;
+    const int per = win_heads(true, small);
+    const dim3 win((unsigned)((T_tok + 15) / 16), (unsigned)((heads + per - 1) / per), kc ? shape.roles : 1u);
+    auto kfn = small ? fill_window_kernel<T, true, true> : fill_window_kernel<T, true, false>;
+    return launch_kernel(kfn, win, dim3(128), 0, s, true, (uint8_t*)q, (uint8_t*)k, (const uint8_t*)v, (uint8_t*)kc, (uint8_t*)vc,
+                         slots, is64, (const long long*)positions, (const uint8_t*)cos_sin, rot_dim, max_pos, T_tok, Hq, H, D, qs, ks,
+                         vs, kbs, khs, num_blocks, write_back);
   }
   const size_t smem = (size_t)kFillWarps * B * D * sizeof(T);
   auto kfn = rotary_fill_kernel<T>;

@@ -296,3 +296,32 @@ def test_moves_right_behind_fills_see_the_new_rows(dtype, scattered):
     torch.cuda.synchronize()
     for k, v, (ko, vo, kb, vb) in zip(keys, values, rows):
         assert torch.equal(ko, k) and torch.equal(vo, v) and torch.equal(kb, k) and torch.equal(vb, v)
+
+
+def _slots_of_runs(rng, t, length, nb, b=16):
+    """t slots in runs of `length` consecutive ones (within a block, at random places), some of them padded or
+    outside the cache."""
+    n = -(-t // length)
+    first = rng.permutation(nb)[:n] * b + rng.integers(0, b - length + 1, size=n)
+    slots = (first[:, None] + np.arange(length)).reshape(-1)[:t]
+    slots[rng.integers(0, t, size=3)] = -1
+    slots[rng.integers(0, t, size=3)] = nb * b + 5
+    return slots
+
+
+# 16 tokens of a window hold the starts of one run, of two (the most that is written run by run), three, and sixteen
+@pytest.mark.parametrize("length", [16, 8, 6, 1])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+@pytest.mark.parametrize("t,h,d", [(4805, 8, 128), (4730, 8, 64), (2401, 16, 80), (1000, 40, 256), (300, 5, 128), (300, 1, 112)])
+def test_fill_large_and_small_batches(dtype, t, h, d, length):
+    """Either side of the batch size from which a CTA takes two heads (2368 windows x heads on 148 SMs) and of the one up to
+    which K and V have CTAs of their own (74)."""
+    nb = -(-t // length) + 3
+    kc, vc, g = _caches(dtype, nb, h, d, 16, 40)
+    slots = _slots_of_runs(np.random.default_rng(41), t, length, nb)
+    qkv = torch.randn((t, 3, h, d), generator=g, device=DEV).to(dtype)
+    _, key, value = qkv.unbind(dim=1)
+    kr, vr = bits(kc).copy(), bits(vc).copy()
+    orc.fill_reference(bits(key), bits(value), kr, vr, np.where(slots < nb * 16, slots, -1))
+    pb.vllm_reshape_and_cache(key, value, kc, vc, torch.tensor(slots, device=DEV))
+    assert np.array_equal(bits(kc), kr) and np.array_equal(bits(vc), vr)

@@ -153,3 +153,34 @@ def test_rotary_rejects_unsupported_shapes():
         pb.vllm_rotary_emb(torch.zeros(2, dtype=torch.int64, device=DEV), q, q.clone(), cs, 128)
     with pytest.raises(RuntimeError):  # dtype mismatch between table and tensors
         pb.vllm_rotary_emb(torch.zeros(2, dtype=torch.int64, device=DEV), q, q.clone(), cs.float(), 128)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("t,hq,hk,d,rot", [(2400, 6, 3, 128, 128), (2368, 6, 5, 64, 32), (800, 3, 20, 128, 64), (600, 4, 2, 256, 128), (40, 3, 2, 80, 80)])
+@pytest.mark.parametrize("length", [16, 3, 1])
+def test_fused_rotary_fill_large_and_small_batches(dtype, t, hq, hk, d, rot, length):
+    """Whole blocks, short runs and lone slots, either side of the batch size from which a CTA takes four heads (888
+    windows x heads on 148 SMs) and of the one up to which q, K and V have CTAs of their own (49)."""
+    b, max_pos = 16, 500
+    nb = -(-t // length) + 2
+    rng = np.random.default_rng(50)
+    slots = (rng.permutation(nb)[:-(-t // length), None] * b + np.arange(length)).reshape(-1)[:t]
+    g = torch.Generator(device=DEV).manual_seed(51)
+    x = 16 // torch.empty((), dtype=dtype).element_size()
+    kc = torch.randn((nb, hk, d // x, b, x), generator=g, device=DEV).to(dtype)
+    vc = torch.randn((nb, hk, d, b), generator=g, device=DEV).to(dtype)
+    qkv = torch.randn((t, (hq + 2 * hk) * d), generator=g, device=DEV).to(dtype)
+    q, k, v = qkv.split([hq * d, hk * d, hk * d], dim=-1)
+    positions = torch.randint(0, max_pos, (t,), generator=g, device=DEV)
+    cs = cos_sin_table(max_pos, rot, dtype)
+    wq, wk = orc.rotary_neox_reference(positions.cpu().numpy(), q.cpu().double().numpy(), k.cpu().double().numpy(),
+                                       cs.cpu().double().numpy(), d)
+    kr, vr = bits(kc).copy(), bits(vc).copy()
+    pb.rotary_reshape_and_cache(positions, q, k, v, kc, vc, torch.tensor(slots, device=DEV), cs, d)
+    assert_rotated(q, wq, dtype, "query")
+    k_back, v_back = (torch.zeros((t, hk, d), dtype=dtype, device=DEV) for _ in range(2))
+    pb.gather_cached_kv(k_back, v_back, kc, vc, torch.tensor(slots, device=DEV))
+    assert_rotated(k_back.view(t, -1), wk, dtype, "cached key")
+    assert np.array_equal(bits(v_back.view(t, -1)), bits(v))
+    orc.fill_reference(bits(k_back), bits(v_back), kr, vr, slots)  # nothing but the addressed slots changed
+    assert np.array_equal(bits(kc), kr) and np.array_equal(bits(vc), vr)
