@@ -619,12 +619,20 @@ __global__ void __launch_bounds__(128) fill_window_kernel(
   }
 }
 
-// dest[dest_idx[i]] = cache row at slot src_slots[i], block size 16: a CTA takes the runs of slots that
-// start among 16 entries of the list, one warp per (run, head). What bounds it is memory: a V tile's
-// 32-byte rows hold 16 tokens, so a warp per (token, head) fetched every tile sixteen times (from L2) in
-// two-byte loads; here it is read once with 16-byte loads and turned in shared memory. K moves as 16-byte
-// chunks, two neighbouring ones of a token per instruction, so that reads and writes are whole sectors.
-// K and V of 8090 tokens x 32 heads x 128 (fp16, 265 MB read and written): 127 -> 57 us, 4.6 TB/s.
+// dest[dest_idx[i]] = cache row at slot src_slots[i], block size 16: a CTA takes 16 entries of the list and a few
+// heads. What bounds it is memory.
+//   K: a warp per head, a pair of lanes per entry: 16-byte chunks, two neighbouring ones of a token per
+//     instruction, so that reads and writes are whole sectors (consecutive slots: neighbouring cells).
+//   V: a tile's 32-byte rows hold 16 tokens, so a warp per (token, head) fetches a tile sixteen times (from L2)
+//     in two-byte loads. The runs of consecutive slots that start among the entries are read once, a warp per (run,
+//     head), with 16-byte loads, and turned in shared memory. Short runs (scattered slots): a warp per (token, head)
+//     after all, four of them at a time, because a whole tile for a few tokens is work in vain (2000 tokens x 32
+//     heads, runs of eleven: fp16 11.8 us, by elements 16; of five 16 and 20, fp32 35 and 52; of three 22 and 19).
+// K and V of 8090 tokens x 32 heads x 128 in whole blocks (fp16, 265 MB read and written): 127 -> 57 us, 4.6 TB/s.
+// 1024 scattered tokens x 32 heads: K 5.8 us, V 13.6 (a warp per run for all of them: 18 and 34; a warp per (token,
+// head): 8.8 and 13.1). In fp32 V takes 70, and 33 with a warp per (token, head) each in a CTA of their own.
+constexpr int kMeanRunMove = 4;  // V moves by runs from this mean length on
+
 template <int E, bool IS_V>
 __global__ void __launch_bounds__(128) move_runs_kernel(
     const uint8_t* cache, uint8_t* dest, const long long* src_slots,
@@ -636,6 +644,7 @@ __global__ void __launch_bounds__(128) move_runs_kernel(
   extern __shared__ __align__(16) uint8_t smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const long long first = (long long)blockIdx.x * 16;
+  const int h0 = blockIdx.y * heads_per_cta, nh = min(heads_per_cta, H - h0);
   pdl_wait();
   pdl_trigger();
   const long long my = first - 1 + lane;
@@ -647,10 +656,61 @@ __global__ void __launch_bounds__(128) move_runs_kernel(
     if (slot < 0 || slot >= num_blocks * B) slot = -1;
     di = -1;  // this entry is skipped
   }
+  if (!IS_V) {
+    const int nch = D / kVec;
+    const long long s = __shfl_sync(0xffffffffu, slot, 1 + (lane >> 1)), to = __shfl_sync(0xffffffffu, di, 1 + (lane >> 1));
+    if (s < 0 || to < 0) return;
+    for (int h = h0 + warp; h < h0 + nh; h += 4) {
+      const uint4* cell = reinterpret_cast<const uint4*>(cache + ((size_t)(s >> 4) * kbs + (size_t)h * khs) * E) + (s & 15);
+      uint4* row = reinterpret_cast<uint4*>(dest + ((size_t)to * dest_stride + (size_t)h * D) * E);
+      for (int base = lane & 1; base < nch; base += 16) {
+        uint4 v[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+          if (base + 2 * u < nch) v[u] = load16(cell + (size_t)(base + 2 * u) * B);
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+          if (base + 2 * u < nch) row[base + 2 * u] = v[u];
+      }
+    }
+    return;
+  }
   const unsigned cont = run_continues(slot);
   const unsigned starts = ~cont & __ballot_sync(0xffffffffu, slot >= 0) & 0x1fffeu;  // entries first .. first + 15
+  if (starts == 0) return;
   const int n_runs = __popc(starts);
-  const int h0 = blockIdx.y * heads_per_cta, nh = min(heads_per_cta, H - h0);
+  using elem_t = typename ElemOf<E>::type;
+  // lanes [lo, hi) hold the entries of those runs
+  const int last = 31 - __clz(starts), lo = __ffs(starts) - 1, hi = last + run_length(cont, last);
+  if (hi - lo < kMeanRunMove * n_runs) {
+    constexpr int kBatch = 4, kSteps = 4;  // kSteps x 32 elements of a row
+    const int n_pairs = (hi - lo) * nh;
+    for (int p0 = warp; p0 < n_pairs; p0 += 4 * kBatch) {
+      const uint8_t* src[kBatch];
+      uint8_t* row[kBatch];
+#pragma unroll
+      for (int u = 0; u < kBatch; ++u) {
+        const int q = min(p0 + 4 * u, n_pairs - 1), l = lo + q / nh, h = h0 + q % nh;
+        const long long s = __shfl_sync(0xffffffffu, slot, l), to = __shfl_sync(0xffffffffu, di, l);
+        src[u] = (p0 + 4 * u < n_pairs && s >= 0 && to >= 0) ? cache + ((size_t)(s >> 4) * kbs + (size_t)h * khs + (s & 15)) * E : nullptr;
+        row[u] = dest + ((size_t)to * dest_stride + (size_t)h * D) * E;
+      }
+      for (int d0 = lane; d0 < D; d0 += kSteps * 32) {
+        elem_t e[kBatch][kSteps];
+#pragma unroll
+        for (int u = 0; u < kBatch; ++u)
+#pragma unroll
+          for (int r = 0; r < kSteps; ++r)
+            if (src[u] && d0 + r * 32 < D) e[u][r] = load_elem<elem_t>(src[u] + (size_t)(d0 + r * 32) * B * E);
+#pragma unroll
+        for (int u = 0; u < kBatch; ++u)
+#pragma unroll
+          for (int r = 0; r < kSteps; ++r)
+            if (src[u] && d0 + r * 32 < D) reinterpret_cast<elem_t*>(row[u])[d0 + r * 32] = e[u][r];
+      }
+    }
+    return;
+  }
   const int words = D * E / 4, pitch = words + 2;  // (two words of padding spread the columns over the banks)
   uint32_t* tile = reinterpret_cast<uint32_t*>(smem) + (size_t)warp * B * pitch;
   for (int task = warp; task < n_runs * nh; task += 4) {
@@ -660,64 +720,44 @@ __global__ void __launch_bounds__(128) move_runs_kernel(
     const long long s0 = __shfl_sync(0xffffffffu, slot, at);
     const int off = (int)(s0 & 15);
     const uint8_t* src = cache + ((size_t)(s0 >> 4) * kbs + (size_t)h * khs) * E;
-    if (IS_V) {
-      // 16-byte chunk: kVec tokens of one d; chunks without a token of the run are left out
-      if (E == 2) {  // rows d, d + 1 and eight tokens: words (token, d pair)
-        const int half = lane & 1;
-        if (half * 8 < off + run && half * 8 + 8 > off) {
+    // 16-byte chunk: kVec tokens of one d; chunks without a token of the run are left out
+    if (E == 2) {  // rows d, d + 1 and eight tokens: words (token, d pair)
+      const int half = lane & 1;
+      if (half * 8 < off + run && half * 8 + 8 > off) {
 #pragma unroll 4
-          for (int p = lane >> 1; p < D / 2; p += 16) {
-            const uint4 a = load16(src + (size_t)p * 64 + half * 16);
-            const uint4 b = load16(src + (size_t)p * 64 + 32 + half * 16);
-            const uint32_t av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
+        for (int p = lane >> 1; p < D / 2; p += 16) {
+          const uint4 a = load16(src + (size_t)p * 64 + half * 16);
+          const uint4 b = load16(src + (size_t)p * 64 + 32 + half * 16);
+          const uint32_t av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              tile[(half * 8 + 2 * j) * pitch + p] = __byte_perm(av[j], bv[j], 0x5410);
-              tile[(half * 8 + 2 * j + 1) * pitch + p] = __byte_perm(av[j], bv[j], 0x7632);
-            }
-          }
-        }
-      } else {
-        const int quarter = lane & 3;
-        if (quarter * 4 < off + run && quarter * 4 + 4 > off) {
-#pragma unroll 4
-          for (int d = lane >> 2; d < D; d += 8) {
-            const uint4 a = load16(src + (size_t)d * 64 + quarter * 16);
-            tile[(quarter * 4 + 0) * pitch + d] = a.x;
-            tile[(quarter * 4 + 1) * pitch + d] = a.y;
-            tile[(quarter * 4 + 2) * pitch + d] = a.z;
-            tile[(quarter * 4 + 3) * pitch + d] = a.w;
+          for (int j = 0; j < 4; ++j) {
+            tile[(half * 8 + 2 * j) * pitch + p] = __byte_perm(av[j], bv[j], 0x5410);
+            tile[(half * 8 + 2 * j + 1) * pitch + p] = __byte_perm(av[j], bv[j], 0x7632);
           }
         }
       }
-      __syncwarp();
-      for (int i = 0; i < run; ++i) {
-        const long long to = __shfl_sync(0xffffffffu, di, at + i);
-        if (to < 0) continue;
-        uint2* row = reinterpret_cast<uint2*>(dest + ((size_t)to * dest_stride + (size_t)h * D) * E);
-        const uint2* from = reinterpret_cast<const uint2*>(tile + (off + i) * pitch);
-        for (int w = lane; w < words / 2; w += 32) row[w] = from[w];
-      }
-      __syncwarp();
     } else {
-      const int i = lane >> 1, nch = D / kVec;
-      const long long to = __shfl_sync(0xffffffffu, di, min(at + i, 31));
-      const bool live = i < run && to >= 0;
-      const uint4* cell = reinterpret_cast<const uint4*>(src) + off + i;
-      uint4* row = reinterpret_cast<uint4*>(dest + ((size_t)(live ? to : 0) * dest_stride + (size_t)h * D) * E);
-      if (live) {
-        for (int base = lane & 1; base < nch; base += 16) {
-          uint4 v[8];
-#pragma unroll
-          for (int u = 0; u < 8; ++u)
-            if (base + 2 * u < nch) v[u] = load16(cell + (size_t)(base + 2 * u) * B);
-#pragma unroll
-          for (int u = 0; u < 8; ++u)
-            if (base + 2 * u < nch) row[base + 2 * u] = v[u];
+      const int quarter = lane & 3;
+      if (quarter * 4 < off + run && quarter * 4 + 4 > off) {
+#pragma unroll 4
+        for (int d = lane >> 2; d < D; d += 8) {
+          const uint4 a = load16(src + (size_t)d * 64 + quarter * 16);
+          tile[(quarter * 4 + 0) * pitch + d] = a.x;
+          tile[(quarter * 4 + 1) * pitch + d] = a.y;
+          tile[(quarter * 4 + 2) * pitch + d] = a.z;
+          tile[(quarter * 4 + 3) * pitch + d] = a.w;
         }
       }
-      __syncwarp();
     }
+    __syncwarp();
+    for (int i = 0; i < run; ++i) {
+      const long long to = __shfl_sync(0xffffffffu, di, at + i);
+      if (to < 0) continue;
+      uint2* row = reinterpret_cast<uint2*>(dest + ((size_t)to * dest_stride + (size_t)h * D) * E);
+      const uint2* from = reinterpret_cast<const uint2*>(tile + (off + i) * pitch);
+      for (int w = lane; w < words / 2; w += 32) row[w] = from[w];
+    }
+    __syncwarp();
   }
 }
 
@@ -958,10 +998,13 @@ int pb_move_tokens_from_blocked_cache(const void* cache, void* dest, const int64
   if (!aligned16(cache) || !aligned16(dest) || dest_stride % vec || kv_block_stride % vec ||
       kv_head_stride % vec)
     return PB_ERR_INVALID_ARG;
-  // Block size 16, the size of the engine's caches: runs of slots (comment of the kernel). Four heads per
-  // CTA, one per warp (eight: 69 us instead of 57 for K and V of 8090 tokens x 32 heads). Head sizes beyond 256 and other block sizes take the
-  // warp per (token, head).
-  if (block_size == 16 && head_size <= 256) {
+  // Block size 16, the size of the engine's caches: a CTA per 16 entries (comment of the kernel) and four heads,
+  // one per warp (eight: 69 us instead of 57 for K and V of 8090 tokens x 32 heads). A short list is bound by
+  // latency, and there a warp per (token, head) is as fast or faster: V up to 8192 pairs (256 tokens x 32 heads in
+  // whole blocks 4.5 us against 4.8, 16 tokens 2.4 against 4.7; 2048 x 8 heads 6.4 against 5.1), K up to 4096 (64
+  // tokens x 32 heads in fp32 2.8 against 3.7, 256 tokens 4.2 against 3.8). Head sizes beyond 256 and other block
+  // sizes take that kernel for everything.
+  if (block_size == 16 && head_size <= 256 && num_tokens * num_heads > (is_value ? 8192 : 4096)) {
     const int heads_per_cta = 4;
     const dim3 runs_grid((unsigned)((num_tokens + 15) / 16), (unsigned)((num_heads + heads_per_cta - 1) / heads_per_cta));
     const size_t smem = is_value ? (size_t)4 * 16 * (head_size * E / 4 + 2) * 4 : 0;

@@ -325,3 +325,23 @@ def test_fill_large_and_small_batches(dtype, t, h, d, length):
     orc.fill_reference(bits(key), bits(value), kr, vr, np.where(slots < nb * 16, slots, -1))
     pb.vllm_reshape_and_cache(key, value, kc, vc, torch.tensor(slots, device=DEV))
     assert np.array_equal(bits(kc), kr) and np.array_equal(bits(vc), vr)
+
+
+@pytest.mark.parametrize("length", [16, 8, 6, 1])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+@pytest.mark.parametrize("t,h,d", [(2731, 3, 128), (2730, 3, 128), (1366, 3, 128), (1365, 3, 64), (1000, 9, 80), (2051, 4, 256)])
+def test_moves_large_and_small(dtype, t, h, d, length):
+    """Either side of the 8192 (token, head) pairs from which values move by runs and of the 4096 for keys, for runs of every kind."""
+    nb = -(-t // length) + 3
+    kc, vc, g = _caches(dtype, nb, h, d, 16, 42)
+    rng = np.random.default_rng(43)
+    src = _slots_of_runs(rng, t, length, nb)
+    dst = rng.permutation(t + 10)[:t]
+    dst[rng.integers(0, t, size=2)] = -1
+    kd, vd = (torch.randn((t + 10, h, d), generator=g, device=DEV).to(dtype) for _ in range(2))
+    ke, ve = bits(kd).copy(), bits(vd).copy()
+    ok = (src >= 0) & (src < nb * 16) & (dst >= 0)
+    ke[dst[ok]], ve[dst[ok]] = orc.gather_reference(bits(kc), bits(vc), src[ok])
+    pb.move_tokens_from_blocked_k_cache(kc, kd, torch.tensor(src, device=DEV), torch.tensor(dst, device=DEV))
+    pb.move_tokens_from_blocked_v_cache(vc, vd, torch.tensor(src, device=DEV), torch.tensor(dst, device=DEV))
+    assert np.array_equal(bits(kd), ke) and np.array_equal(bits(vd), ve)
