@@ -18,82 +18,55 @@ constexpr int kPairLanes = 16;                 // lanes that share one (row, hea
 constexpr int kPairsPerWarp = 32 / kPairLanes;  // two (row, head) pairs per warp: twice the loads in flight
 constexpr int kPairs = kMergeWarps * kPairsPerWarp;  // heads a CTA works on at once
 constexpr int kMaxHeadsPerCta = kMergeWarps * 32;    // one thread each finds a head's partials
-constexpr int kManyRows = 1024;                      // prefill batches from here on: a CTA takes up to kMaxHeadsPerCta heads of a row
+constexpr int kManyRows = 1024;                      // prefill rows from which a CTA walks up to kMaxHeadsPerCta heads of a row
 
-// dense_cta_of_tile, with a 32-bit division wherever the product fits: the 64-bit one is a routine of some
-// hundred instructions, and every (row, head) asks twice.
+// dense_cta_of_tile without a 64-bit division (a routine of some hundred instructions, and every (row, head) asks
+// twice): the quotient is at most kMaxSMs, so an estimate in fp32 is off by one at most, and the remainder says so.
 __device__ __forceinline__ int cta_of_tile(long long g, long long total, int ctas) {
   const int c = dense_active_ctas(total, ctas);
-  if (total < (1ll << 24)) return (int)(((uint32_t)(g + 1) * (uint32_t)c + (uint32_t)(total - 1)) / (uint32_t)total) - 1;
-  return dense_cta_of_tile(g, total, ctas);
+  const long long num = (g + 1) * c + total - 1;
+  int q = (int)__fdividef((float)num, (float)total);
+  const long long rest = num - q * total;
+  q += rest >= total ? 1 : rest < 0 ? -1 : 0;
+  return q - 1;
 }
-static_assert((1ull << 24) * (kMaxSMs + 1) < (1ull << 32), "the 32-bit product must fit");
 
-// kMany == false: a CTA per eight heads of a row; the lanes of a (row, head) find its partials for themselves.
-// kMany == true (prefill): a CTA per row (and 128 heads) walks its heads eight at a time. How many
-// partials a head has is worked out by one thread per head; a row that the dense kernel has finished leaves at
-// once. (With a CTA per eight pairs, all lanes dividing, a batch of ten thousand prefill rows spent 100 us on
-// finding out that there was nothing to do. For few rows the detour through shared memory costs 1.5 us.)
-template <typename T, int D, bool kMany>
-__global__ void __launch_bounds__(kMergeWarps * 32) merge_kernel(const AttnDev d, const int heads_per_cta) {
-  // (kMany) partials of each head: prefix, segment, outer prefix; w: 1 = finished by the dense kernel
-  extern __shared__ int4 parts_of[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int sub = lane % kPairLanes;  // position inside the pair's lane group
-  const int H = d.num_heads;
-  const int per_row = (H + heads_per_cta - 1) / heads_per_cta;  // CTAs of a row, next to each other
-  const int row = blockIdx.x / per_row, h_lo = (blockIdx.x - row * per_row) * heads_per_cta, h_hi = min(H, h_lo + heads_per_cta);
-  // The planner's output (row_info, dense items, header) is older than the attention kernels of
-  // this call, so it is read while they still run; only then wait for their partials.
-  const RowInfo info = d.row_info[row];
-  const long long total = d.hdr[kHdrDnTiles];
-  const int dctas = dense_ctas_of(d);
-  // partials of the row: [prefix][causal segment][suffix]; a dense stage leaves one partial per
-  // CTA that touched the (row tile, head), the single-query kernel one per chunk
-  auto parts = [&](int head) {
-    auto dense_parts = [&](int dn) {
-      const int nt = d.dn_items[dn].nt, fixed = d.dn_items[dn].fixed;
-      const long long g0 = (long long)d.dn_items[dn].tile_base + (long long)head * (fixed + nt) + fixed;
-      return cta_of_tile(g0 + nt - 1, total, dctas) - cta_of_tile(g0, total, dctas) + 1;
-    };
-    int4 p;
-    p.x = (info.dn >= 0) ? dense_parts(info.dn) : info.np_sq;
-    p.y = (info.seg_dn >= 0) ? dense_parts(info.seg_dn) : info.nc_sq;
-    p.z = (info.odn >= 0) ? dense_parts(info.odn) : info.onp_sq;  // outer-prefix partials
-    // rows the dense kernel finished by itself (their only partial, held whole by one CTA): nothing to do
-    const int only = (info.dn >= 0 && p.x == 1 && p.y == 0) ? info.dn : (info.seg_dn >= 0 && p.y == 1 && p.x == 0) ? info.seg_dn : -1;
-    p.w = (only >= 0 && info.nsc == 0 && p.z == 0 && dense_direct_ok(d, d.dn_items[only])) ? 1 : 0;
-    return p;
+// Partials of one (row, head): [prefix][causal segment][suffix][outer prefix]; a dense stage leaves one partial per
+// CTA that touched the (row tile, head), the single-query kernel one per chunk (suffix: info.nsc).
+struct PartCounts {
+  int prefix, segment, outer;
+  bool direct;  // finished by the dense kernel (its only partial, held whole by one CTA): nothing to merge
+};
+__device__ __forceinline__ PartCounts count_parts(const AttnDev& d, const RowInfo& info, long long total, int dctas, int head) {
+  auto dense_parts = [&](int dn) {
+    const int nt = d.dn_items[dn].nt, fixed = d.dn_items[dn].fixed;
+    const long long g0 = (long long)d.dn_items[dn].tile_base + (long long)head * (fixed + nt) + fixed;
+    return cta_of_tile(g0 + nt - 1, total, dctas) - cta_of_tile(g0, total, dctas) + 1;
   };
-  int4 mine = make_int4(0, 0, 0, 0);
-  bool any_open = true;
-  if (kMany) {
-    bool open = false;
-    if ((int)threadIdx.x < h_hi - h_lo) {
-      mine = parts(h_lo + threadIdx.x);
-      parts_of[threadIdx.x] = mine;
-      open = mine.w == 0;
-    }
-    any_open = __syncthreads_or(open);
-  } else {
-    const int head = h_lo + warp * kPairsPerWarp + lane / kPairLanes;
-    if (head < h_hi) mine = parts(head);
-  }
-  pdl_wait();  // every partial of the prefix and suffix stages is complete and visible
-  if (blockIdx.x == 0 && threadIdx.x == 0) d.hdr[kHdrSqCounter] = 0;  // ready for the next layer call
-  // A call whose kernels recorded a fault (a wait that ran out, an index outside the cache, a list
-  // that did not fit) has results that cannot be trusted: every output row becomes NaN, so that the
-  // fault cannot pass unnoticed into the sampler even if nobody reads the status word.
-  const bool poison = __ldcg(&d.hdr[kHdrStatus]) != kStatusOk;
-  if (kMany && !any_open && !poison) return;
-  for (int hb = h_lo; hb < (kMany ? h_hi : h_lo + 1); hb += kPairs) {
-  const int head = hb + warp * kPairsPerWarp + lane / kPairLanes;
-  const bool active = head < h_hi;
-  if (kMany) mine = active ? parts_of[head - h_lo] : make_int4(0, 0, 0, 0);
-  const int np = mine.x, nc = mine.y, no = mine.z;
-  const bool direct = mine.w != 0;
-  const long long idx = (long long)row * H + head;
-  const int n = (active && !direct) ? np + nc + info.nsc + no : 0;
+  PartCounts p;
+  p.prefix = (info.dn >= 0) ? dense_parts(info.dn) : info.np_sq;
+  p.segment = (info.seg_dn >= 0) ? dense_parts(info.seg_dn) : info.nc_sq;
+  p.outer = (info.odn >= 0) ? dense_parts(info.odn) : info.onp_sq;
+  const int only = (info.dn >= 0 && p.prefix == 1 && p.segment == 0)       ? info.dn
+                   : (info.seg_dn >= 0 && p.segment == 1 && p.prefix == 0) ? info.seg_dn
+                                                                           : -1;
+  p.direct = only >= 0 && info.nsc == 0 && p.outer == 0 && dense_direct_ok(d, d.dn_items[only]);
+  return p;
+}
+
+// A call whose kernels recorded a fault (a wait that ran out, an index outside the cache, a list
+// that did not fit) has results that cannot be trusted: every output row becomes NaN, so that the
+// fault cannot pass unnoticed into the sampler even if nobody reads the status word.
+__device__ __forceinline__ bool call_failed(const AttnDev& d) { return __ldcg(&d.hdr[kHdrStatus]) != kStatusOk; }
+
+// Merges the partials of (row, head); the kPairLanes lanes of a (row, head) call it together, both halves of a warp
+// in lockstep (active == false: a half without work).
+template <typename T, int D>
+__device__ __forceinline__ void merge_one(const AttnDev& d, const int row, const int head, const long long idx, const bool active,
+                                          const int nsc, const PartCounts& parts, const bool poison) {
+  const int sub = (threadIdx.x & 31) % kPairLanes;  // position inside the pair's lane group
+  const int np = parts.prefix, nc = parts.segment;
+  const int n = (active && !parts.direct) ? np + nc + nsc + parts.outer : 0;
   int n_warp = n;  // the two pairs of a warp walk their partials in lockstep
 #pragma unroll
   for (int o = kPairLanes; o < 32; o <<= 1) n_warp = max(n_warp, __shfl_xor_sync(0xffffffffu, n_warp, o));
@@ -102,8 +75,8 @@ __global__ void __launch_bounds__(kMergeWarps * 32) merge_kernel(const AttnDev d
   auto part_of = [&](int j) {  // partial ranges of a row: [prefix][segment][suffix][outer prefix]
     if (j < np) return j;
     if (j < np + nc) return d.pparts + (j - np);
-    if (j < np + nc + info.nsc) return d.pparts + d.cparts + (j - np - nc);
-    return d.pparts + d.cparts + d.sparts + (j - np - nc - info.nsc);
+    if (j < np + nc + nsc) return d.pparts + d.cparts + (j - np - nc);
+    return d.pparts + d.cparts + d.sparts + (j - np - nc - nsc);
   };
 
   const bool load_prev = (d.stats_mode & PB_STATS_LOAD) != 0;
@@ -125,7 +98,7 @@ __global__ void __launch_bounds__(kMergeWarps * 32) merge_kernel(const AttnDev d
   for (int o = kPairLanes / 2; o >= 1; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
   // The next kernel in the stream may become resident: every kernel of this library that is launched early
   // waits for this grid's completion before it writes anything to global memory (the planner counts first).
-  if (hb == h_lo) pdl_trigger();
+  pdl_trigger();
 
   float4 o4[kPer];
 #pragma unroll
@@ -171,7 +144,7 @@ __global__ void __launch_bounds__(kMergeWarps * 32) merge_kernel(const AttnDev d
   }
 #pragma unroll
   for (int o = kPairLanes / 2; o >= 1; o >>= 1) L += __shfl_xor_sync(0xffffffffu, L, o);
-  if (!active || (direct && !poison)) continue;
+  if (!active || (parts.direct && !poison)) return;
   if (l_prev > 0.f) {
     const float w = fast_exp2(m_prev - M) * l_prev;
     L += w;
@@ -203,16 +176,68 @@ __global__ void __launch_bounds__(kMergeWarps * 32) merge_kernel(const AttnDev d
     d.qk_max[idx] = M;
     d.exp_sum[idx] = L;
   }
-  }  // heads
+}
+
+// Decode batches and small ones: (row, head) pairs packed over the rows, eight to a CTA; the lanes of a pair find
+// its partials for themselves. A head count that is no multiple of eight leaves no lane idle (a step of 1024 rows x
+// 4 heads over 2048 tokens: 42.4 us with CTAs that end with their row, 41.6 so). Registers decide how many pairs are
+// in flight: 72 are seven CTAs an SM (256 rows x 32 heads: 67.0 us a step with 76 registers, six CTAs, 64.5 so; the
+// headline step of 64 rows, whose merge fits the chip once, 72.1 and 72.4). What only the walk below needs stays out.
+template <typename T, int D>
+__global__ void __launch_bounds__(kMergeWarps * 32) merge_kernel(const AttnDev d) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const long long idx = ((long long)blockIdx.x * kMergeWarps + warp) * kPairsPerWarp + lane / kPairLanes;
+  const int H = d.num_heads;
+  const bool active = idx < (long long)d.num_rows * H;
+  const int row = active ? (int)(idx / H) : 0, head = active ? (int)(idx - (long long)row * H) : 0;
+  // The planner's output (row_info, dense items, header) is older than the attention kernels of
+  // this call, so it is read while they still run; only then wait for their partials.
+  const RowInfo info = d.row_info[row];
+  const PartCounts parts = count_parts(d, info, d.hdr[kHdrDnTiles], dense_ctas_of(d), head);
+  pdl_wait();  // every partial of the prefix and suffix stages is complete and visible
+  if (blockIdx.x == 0 && threadIdx.x == 0) d.hdr[kHdrSqCounter] = 0;  // ready for the next layer call
+  merge_one<T, D>(d, row, head, idx, active, info.nsc, parts, call_failed(d));
+}
+
+// Batches with many prefill rows: a CTA per row (and 128 heads) walks its heads eight at a time. How many partials
+// a head has is worked out by one thread per head; a row that the dense kernel has finished leaves at once. (With a
+// CTA per eight pairs, all lanes dividing, a batch of ten thousand prefill rows spent 100 us on finding out that there
+// was nothing to do. For few rows the detour through shared memory costs 1.5 us.)
+template <typename T, int D>
+__global__ void __launch_bounds__(kMergeWarps * 32) merge_rows_kernel(const AttnDev d, const int heads_per_cta) {
+  extern __shared__ PartCounts parts_of[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int H = d.num_heads;
+  const int per_row = (H + heads_per_cta - 1) / heads_per_cta;  // CTAs of a row, next to each other
+  const int row = blockIdx.x / per_row, h_lo = (blockIdx.x - row * per_row) * heads_per_cta, h_hi = min(H, h_lo + heads_per_cta);
+  const RowInfo info = d.row_info[row];
+  bool open = false;
+  if ((int)threadIdx.x < h_hi - h_lo) {
+    const PartCounts mine = count_parts(d, info, d.hdr[kHdrDnTiles], dense_ctas_of(d), h_lo + threadIdx.x);
+    parts_of[threadIdx.x] = mine;
+    open = !mine.direct;
+  }
+  const bool any_open = __syncthreads_or(open);
+  pdl_wait();  // as above
+  if (blockIdx.x == 0 && threadIdx.x == 0) d.hdr[kHdrSqCounter] = 0;
+  const bool poison = call_failed(d);
+  if (!any_open && !poison) return;
+  for (int hb = h_lo; hb < h_hi; hb += kPairs) {
+    const int head = hb + warp * kPairsPerWarp + lane / kPairLanes;
+    const bool active = head < h_hi;
+    merge_one<T, D>(d, row, head, (long long)row * H + head, active, info.nsc, parts_of[(active ? head : h_lo) - h_lo], poison);
+  }
 }
 
 template <typename T, int D>
 cudaError_t launch_merge_d(const AttnDev& d, cudaStream_t s) {
-  const bool many = d.num_segments > 0 && d.num_rows >= kManyRows;  // (only prefill rows are ever finished before)
-  const int hpc = !many ? kPairs : d.num_heads < kMaxHeadsPerCta ? d.num_heads : kMaxHeadsPerCta;
-  const unsigned grid = (unsigned)((long long)d.num_rows * ((d.num_heads + hpc - 1) / hpc));
-  return many ? launch_kernel(merge_kernel<T, D, true>, grid, kMergeWarps * 32, (size_t)hpc * sizeof(int4), s, true, d, hpc)
-              : launch_kernel(merge_kernel<T, D, false>, grid, kMergeWarps * 32, 0, s, true, d, hpc);
+  if (d.num_segments > 0 && d.num_rows >= kManyRows) {  // (only prefill rows are ever finished before)
+    const int hpc = d.num_heads < kMaxHeadsPerCta ? d.num_heads : kMaxHeadsPerCta;
+    const unsigned grid = (unsigned)((long long)d.num_rows * ((d.num_heads + hpc - 1) / hpc));
+    return launch_kernel(merge_rows_kernel<T, D>, grid, kMergeWarps * 32, (size_t)hpc * sizeof(PartCounts), s, true, d, hpc);
+  }
+  const unsigned grid = (unsigned)(((long long)d.num_rows * d.num_heads + kPairs - 1) / kPairs);
+  return launch_kernel(merge_kernel<T, D>, grid, kMergeWarps * 32, 0, s, true, d);
 }
 
 template <typename T>

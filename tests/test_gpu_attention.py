@@ -815,3 +815,36 @@ def test_lists_that_do_not_fit_are_reported(dense_min_rows):
     out = torch.zeros_like(q)
     call.run(q, out, kc, vc)
     assert call.status() == 3 and torch.isnan(out).all()
+
+
+@pytest.mark.parametrize("new,decode,heads", [([16], 1100, 4), ([1024], 24, 12), ([700, 420], 30, 20), ([1023], 0, 5), ([1100], 0, 130)])
+def test_merge_of_batches_around_its_forms(new, decode, heads):
+    """Few and many prefill rows (the merge's walk over a row's heads), head counts that are no multiple of eight and
+    more than one CTA walks; rows that are finished before the merge beside rows that are not."""
+    plen, n_new = 128, sum(new)
+    up = lambda n: -(-n // 16)
+    rng = np.random.default_rng(80)
+    sl = [0] * n_new + rng.integers(1, 40, size=decode).tolist()
+    nb = up(plen) + sum(up(n) for n in new) + sum(up(n) for n in sl) + 4
+    g = torch.Generator(device=DEV).manual_seed(81)
+    kc = torch.randn((nb, heads, 16, 16, 8), generator=g, device=DEV).half()
+    vc = torch.randn((nb, heads, 128, 16), generator=g, device=DEV).half()
+    q = torch.randn((n_new + decode, heads, 128), generator=g, device=DEV).half()
+    perm = rng.permutation(nb).tolist()
+    deal = lambda n: [perm.pop() for _ in range(up(n))]
+    pad = lambda rows: [r + [0] * (max(map(len, rows + [[0]])) - len(r)) for r in rows]
+    gt, nt, st = [deal(plen)], pad([deal(n) for n in new]), pad([deal(n) for n in sl])
+    i32 = lambda a: torch.tensor(a, dtype=torch.int32, device=DEV)
+    seg_offs = np.cumsum([0] + new).tolist()
+    call = pb.AttentionCall(num_rows=n_new + decode, num_heads=heads, head_size=128, block_size=16, dtype=q.dtype, device=q.device,
+                            suffix_lens=i32(sl), suffix_tables=i32(st), group_row_offsets=i32([0, n_new + decode]),
+                            group_prefix_lens=i32([plen]), group_tables=i32(gt), seg_row_offsets=i32(seg_offs), seg_kv_lens=i32(new),
+                            seg_tables=i32(nt))
+    out = torch.full_like(q, float("nan"))
+    call.run(q, out, kc, vc)
+    assert call.status() == 0 and torch.isfinite(out).all()
+    rows = sorted({0, 1, new[0] - 1, n_new - 1, min(n_new, n_new + decode - 1), n_new + decode - 1, n_new // 2})
+    hs = sorted({0, heads // 2, heads - 1})
+    ref = orc.gold_grouped_attention(q[:, hs].float().cpu(), kc[:, hs].float().cpu(), vc[:, hs].float().cpu(), [0, n_new + decode], [plen],
+                                     gt, sl, st, rows=rows, heads=list(range(len(hs))), seg_row_offsets=seg_offs, seg_kv_lens=new, seg_tables=nt)
+    assert_close_to_oracle(out[rows][:, hs], ref, q.dtype, "merge forms")
