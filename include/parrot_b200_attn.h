@@ -142,8 +142,9 @@ typedef struct pb_attn_params {
   int32_t dense_row_tile;    /* query rows per work item of the tensor-core kernel: 128 (one row tile per
                               * pass; shares a row's exponentials between threads when a group has at most
                               * 64 rows) or 256 (two row tiles share every K/V tile, softmax of one under the
-                              * MMAs of the other: the prefill shape). 0 = chosen from num_rows and
-                              * num_segments: 256 for large batches of prefill requests, else 128.
+                              * MMAs of the other: the prefill shape). 0 = chosen from num_rows,
+                              * num_groups, num_segments and seg_table_stride: 256 for large batches of prefill requests of
+                              * more than 128 tokens each, alone or in prefix groups of 250 rows and more on average, else 128.
                               * Part of the plan. Any other value is an invalid argument. */
   /* scratch */
   void* workspace;

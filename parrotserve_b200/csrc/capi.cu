@@ -1,5 +1,6 @@
 // extern "C" entry points of the attention path: validation, workspace carve-up, launch order.
 // No allocation, no host synchronisation (except pb_read_status), nothing thrown.
+#include <algorithm>
 #include <mutex>
 
 #include "common.cuh"
@@ -202,13 +203,21 @@ int validate_and_bind(const pb_attn_params* p, WsLayout* L, AttnDev* d) {
   // Read by the planner only: the split is part of the plan.
   d->num_sms = sm_count();
   d->dense_ctas = p->dense_ctas > 0 ? (p->dense_ctas < d->num_sms ? p->dense_ctas : d->num_sms) : 0;
+  // Most rows the segments can have: a segment's rows are tokens of its context, and its table holds that.
+  // (The lengths themselves are in device memory; decode rows of the batch must not pass for prefill rows.)
+  d->seg_rows_max = (int32_t)std::min<long long>(p->num_rows, (long long)p->num_segments * p->seg_table_stride * p->block_size);
   // Rows per dense item. Row-tile pairs pay in batches of prefill requests of more than 128 rows each (32 x 140
   // rows, 32 heads: 180 us against 197 with single tiles; 4 x 2192: 439 against 485; under a 512-token
   // prefix 32 x 140: 295 against 338). Requests of at most 128 rows leave half of the pair kernel's softmax
   // threads idle (32 x 128 under that prefix: 238 against 199), and with few rows in all the single tiles
-  // spread over more SMs (1 x 256: 37 against 35; 1 x 1000: 71 against 76).
-  d->dense_row_tile = p->dense_row_tile > 0 ? p->dense_row_tile
-                      : (p->num_segments > 0 && p->num_rows >= 1000 && (long long)p->num_rows > 128ll * p->num_segments) ? 256 : 128;
+  // spread over more SMs (1 x 256: 37 against 35; 1 x 1000: 71 against 76). So do prefix groups with few
+  // decode rows, which also lose the form in which several threads share a row's exponentials (prefix 2048: 32 groups x 32
+  // decode rows with 4 x 300 prefill rows 548 against 470, 16 x 64 with 1 x 2000 446 against 439, 4 x 250 with 1 x 512
+  // 246 against 259): with groups, pairs from 250 rows a group on. Without groups decode rows are no dense work and do not count.
+  const long long dense_rows = p->num_groups > 0 ? p->num_rows : d->seg_rows_max;
+  const bool pairs = p->num_segments > 0 && dense_rows >= 1000 && dense_rows > 128ll * p->num_segments &&
+                     p->num_rows >= 250ll * p->num_groups;
+  d->dense_row_tile = p->dense_row_tile > 0 ? p->dense_row_tile : pairs ? 256 : 128;
   d->q_stride = p->q_stride; d->out_stride = p->out_stride;
   d->out_vec16 = (aligned16(p->out) && (p->out_stride * elem_bytes(p->dtype)) % 16 == 0) ? 1 : 0;
   d->acc_tma = 0;

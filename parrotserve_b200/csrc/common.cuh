@@ -301,6 +301,7 @@ struct AttnDev {            // what the attention kernels read
   const int32_t* outer_tables;
   int32_t num_outer_groups, outer_table_stride;
   int32_t sq_waits_at_start;  // 1: no dense kernel precedes the single-query kernel in this call
+  int32_t seg_rows_max;       // most rows the causal segments can have (prefill rows), from the sizes of their tables
   int32_t dense_row_tile;     // rows per dense item: 128 (one row tile per CTA pass) or 256 (row-tile pairs)
   int32_t acc_tma;            // 1: the dense kernel may write full row tiles of partials with TMA tiled stores
   // new tokens of the step (see pb_attn_params): slot_mapping is the planner's input; key_new /

@@ -231,7 +231,7 @@ __global__ void __launch_bounds__(kMergeWarps * 32) merge_rows_kernel(const Attn
 
 template <typename T, int D>
 cudaError_t launch_merge_d(const AttnDev& d, cudaStream_t s) {
-  if (d.num_segments > 0 && d.num_rows >= kManyRows) {  // (only prefill rows are ever finished before)
+  if (d.seg_rows_max >= kManyRows) {  // (only prefill rows are ever finished before; decode rows do not count)
     const int hpc = d.num_heads < kMaxHeadsPerCta ? d.num_heads : kMaxHeadsPerCta;
     const unsigned grid = (unsigned)((long long)d.num_rows * ((d.num_heads + hpc - 1) / hpc));
     return launch_kernel(merge_rows_kernel<T, D>, grid, kMergeWarps * 32, (size_t)hpc * sizeof(PartCounts), s, true, d, hpc);

@@ -848,3 +848,42 @@ def test_merge_of_batches_around_its_forms(new, decode, heads):
     ref = orc.gold_grouped_attention(q[:, hs].float().cpu(), kc[:, hs].float().cpu(), vc[:, hs].float().cpu(), [0, n_new + decode], [plen],
                                      gt, sl, st, rows=rows, heads=list(range(len(hs))), seg_row_offsets=seg_offs, seg_kv_lens=new, seg_tables=nt)
     assert_close_to_oracle(out[rows][:, hs], ref, q.dtype, "merge forms")
+
+
+def _planned_header(new, decode, groups, prefix=256, suffix=16, heads=1, **tuning):
+    """The header the planner leaves for a batch of prefills (`new` tokens each, in the first group) and `decode` rows
+    spread evenly over the groups: [2] dense items, [5] CTAs of the dense kernel."""
+    i32 = lambda a: torch.tensor(a, dtype=torch.int32, device=DEV)
+    rows = sum(new) + decode
+    up = lambda n: -(-n // 16)
+    meta = dict(suffix_lens=i32([0] * sum(new) + [suffix] * decode), suffix_tables=torch.zeros((rows, up(suffix)), dtype=torch.int32, device=DEV))
+    if groups:
+        counts = [decode * (g + 1) // groups - decode * g // groups for g in range(groups)]
+        counts[0] += sum(new)
+        meta.update(group_row_offsets=i32(np.cumsum([0] + counts).tolist()), group_prefix_lens=i32([prefix] * groups),
+                    group_tables=torch.zeros((groups, up(prefix)), dtype=torch.int32, device=DEV))
+    if new:
+        meta.update(seg_row_offsets=i32(np.cumsum([0] + new).tolist()), seg_kv_lens=i32(new),
+                    seg_tables=torch.zeros((len(new), up(max(new))), dtype=torch.int32, device=DEV))
+    call = pb.AttentionCall(num_rows=rows, num_heads=heads, head_size=128, block_size=16, dtype=torch.float16, device=torch.device(DEV),
+                            **meta, **tuning)
+    q = torch.zeros((rows, heads, 128), dtype=torch.float16, device=DEV)
+    kc = torch.zeros((4, heads, 16, 16, 8), dtype=torch.float16, device=DEV)
+    vc = torch.zeros((4, heads, 128, 16), dtype=torch.float16, device=DEV)
+    call.plan(q, torch.empty_like(q), kc, vc)
+    assert call.status() == 0
+    return call.workspace[:256].view(torch.int32).tolist()
+
+
+@pytest.mark.parametrize("new,decode,groups,tile", [
+    ([200], 1000, 0, 128),         # decode rows without a group are no dense work
+    ([100] * 16, 400, 1, 128), ([16], 1000, 1, 256),
+    ([1000], 0, 0, 256), ([999], 0, 0, 128), ([100] * 10 + [130], 0, 0, 128), ([140] * 8, 0, 0, 256),
+    ([1024] * 2, 240, 1, 256),     # long prefills and decodes under one prompt
+    ([512] * 2, 512, 16, 128),     # the decode rows of small groups
+    ([512] * 2, 512, 4, 256), ([16], 1000, 4, 256),
+])
+def test_default_row_tile(new, decode, groups, tile):
+    """Row-tile pairs are the default for batches of long prefills in large groups only (dense items of the plan)."""
+    items = {t: _planned_header(new, decode, groups, dense_row_tile=t)[2] for t in (0, 128, 256)}
+    assert items[128] != items[256] and items[0] == items[tile]
