@@ -47,7 +47,7 @@ def _digest(paths) -> str:
 
 
 def build(force: bool = False, verbose: bool = False) -> Path:
-    deps = [CSRC / s for s in SOURCES] + list(CSRC.glob("*.cuh")) + [PKG.parent / "include" / "parrot_b200_attn.h"]
+    deps = [CSRC / s for s in SOURCES] + list(CSRC.glob("*.cuh")) + list(CSRC.glob("*.h")) + [PKG.parent / "include" / "parrot_b200_attn.h"]
     stamp = OBJ_DIR / "stamp.txt"
     digest = _digest(deps)
     if not force and OUT.exists() and stamp.exists() and stamp.read_text() == digest:

@@ -45,6 +45,7 @@
 #include <cuda.h>
 #include <string.h>
 
+#include "arg_table.h"
 #include "common.cuh"
 #include "dense_common.cuh"
 
@@ -625,39 +626,30 @@ EncodeTiledFn encode_tiled_fn() {
 
 // cuTensorMapEncodeTiled is a pure function of its arguments; a layer call needs four maps and a
 // model runs the same shapes over a set of buffers (the caches of its layers) iteration after iteration, so
-// the encoded maps of this thread's calls are kept in a table indexed by a hash of ALL their arguments and
-// compared in full. (A list of 64, searched from the front, was too short for a model of 32 layers, whose
-// caches and outputs are 66 maps: every lookup went through all of it and then encoded the map again.)
+// the encoded maps of this thread's calls are kept in a table (arg_table.h) and found by all their arguments:
+// a model of 32 layers has 66 maps, one of 80 layers 162, and from the second iteration on none is encoded again.
 struct MapKey {
   int type, rank, swizzle, promo;
   const void* base;
   cuuint64_t dims[4], strides[3];
   cuuint32_t box[4];
 };
-struct MapSlot { MapKey key; CUtensorMap map; bool used; };
-constexpr int kMapSlots = 256;
 
 CUresult encode_cached(EncodeTiledFn enc, CUtensorMap* out, CUtensorMapDataType type, int rank, const void* base,
                        const cuuint64_t* dims, const cuuint64_t* strides, const cuuint32_t* box,
                        CUtensorMapSwizzle swizzle, CUtensorMapL2promotion promo) {
-  thread_local MapSlot slots[kMapSlots] = {};
+  thread_local ArgTable<MapKey, CUtensorMap, 256, 64> table;
   MapKey k;
   memset(&k, 0, sizeof(k));
   k.type = (int)type; k.rank = rank; k.swizzle = (int)swizzle; k.promo = (int)promo; k.base = base;
   for (int i = 0; i < rank; ++i) { k.dims[i] = dims[i]; k.box[i] = box[i]; }
   for (int i = 0; i + 1 < rank; ++i) k.strides[i] = strides[i];
-  uint64_t words[sizeof(MapKey) / 8], h = 0;
-  static_assert(sizeof(MapKey) % 8 == 0, "hashed in words");
-  memcpy(words, &k, sizeof(k));
-  for (uint64_t w : words) h = (h ^ w) * 0x9e3779b97f4a7c15ull, h ^= h >> 32;
-  MapSlot& sl = slots[h % kMapSlots];
-  if (sl.used && memcmp(&sl.key, &k, sizeof(k)) == 0) { *out = sl.map; return CUDA_SUCCESS; }
+  uint64_t hash;
+  if (const CUtensorMap* known = table.find(k, &hash)) { *out = *known; return CUDA_SUCCESS; }
   const cuuint32_t estr[4] = {1, 1, 1, 1};
   const CUresult r = enc(out, type, (cuuint32_t)rank, const_cast<void*>(base), dims, strides, box, estr,
                          CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, promo, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r == CUDA_SUCCESS) {
-    sl.key = k; sl.map = *out; sl.used = true;
-  }
+  if (r == CUDA_SUCCESS) table.put(k, hash, *out);
   return r;
 }
 

@@ -604,3 +604,47 @@ def test_two_rank_head_sharding_under_gloo(tmp_path):
                               stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True) for r in range(2)]
     outs = [p.communicate(timeout=240)[0] for p in procs]
     assert all(p.returncode == 0 for p in procs), "\n".join(outs)
+
+
+def test_table_of_tensor_maps_keeps_every_map_of_a_model(tmp_path):
+    """csrc/arg_table.h, compiled here: the maps of models with 32, 40 and 80 layers (two caches each, laid out as one
+    allocation or as many, at many addresses) are each computed once; with more keys than slots a lookup still
+    returns the value of its own key."""
+    src = tmp_path / "table.cpp"
+    src.write_text(r"""
+#include "arg_table.h"
+#include <stdio.h>
+#include <random>
+struct Key { int kind, rank; const void* base; uint64_t dims[4], strides[3]; unsigned box[4]; };
+struct Value { uint64_t of; char map[120]; };
+int main() {
+  std::mt19937_64 rng(1);
+  int computed_again = 0, wrong = 0;
+  for (int trial = 0; trial < 300; ++trial)
+    for (int layers : {32, 40, 80, 400}) {
+      static pb::ArgTable<Key, Value, 256, 64> table;
+      table = {};
+      const uint64_t bytes = 512 * (1 + rng() % 100000), base = 0x7f0000000000ull + 512 * (rng() % 1000000);
+      for (int pass = 0; pass < 3; ++pass)
+        for (int i = 0; i < 2 * layers + 2; ++i) {
+          Key k;
+          memset(&k, 0, sizeof(k));
+          k.kind = i >= 2 * layers; k.rank = 4; k.dims[0] = 16; k.dims[1] = 128; k.strides[0] = 32;
+          const uint64_t at = (trial & 1) ? base + i * bytes : base + (i / 2) * bytes + (i & 1) * (bytes * layers + (2 << 20));
+          k.base = reinterpret_cast<const void*>(at);
+          uint64_t hash;
+          const Value* v = table.find(k, &hash);
+          if (v && v->of != at + k.kind) ++wrong;
+          if (v) continue;
+          if (pass && layers <= 80) ++computed_again;
+          Value mine = {at + k.kind, {}};
+          table.put(k, hash, mine);
+        }
+    }
+  printf("%d %d\n", computed_again, wrong);
+}
+""")
+    csrc = ROOT / "parrotserve_b200" / "csrc"
+    exe = tmp_path / "table"
+    subprocess.run(["g++", "-O1", "-std=c++17", "-Wall", "-Werror", f"-I{csrc}", str(src), "-o", str(exe)], check=True)
+    assert subprocess.run([str(exe)], check=True, capture_output=True, text=True).stdout.split() == ["0", "0"]
