@@ -37,7 +37,7 @@ def _prepare(out, query, key_cache, value_cache, head_mapping, block_tables, con
     ws = Workspace.get(query.device, nbytes)
     tail = (block_size, max_blocks * block_size, num_seqs, num_heads, hkv, head_size, max_blocks, query.stride(0),
             kbs, khs, nb, _dtype_code(query), ws.data_ptr(), ws.numel(), _stream(query))
-    return block_tables, tail
+    return (block_tables, ws), tail  # both are held until the call is enqueued
 
 
 def single_query_cached_kv_attention(out, query, key_cache, value_cache, head_mapping, scale, block_tables,
@@ -47,7 +47,7 @@ def single_query_cached_kv_attention(out, query, key_cache, value_cache, head_ma
     ``block_nums[seq]`` table entries, masking tokens at or beyond ``context_lens[seq]``
     (csrc/attention/attention_kernels.cu:159-162,203); here ceil(context_len / block_size) blocks
     are walked, the same attention for every consistent ``block_nums``, so both tensors are dropped."""
-    bt, tail = _prepare(out, query, key_cache, value_cache, head_mapping, block_tables, context_lens, block_size, alibi_slopes)
+    (bt, ws), tail = _prepare(out, query, key_cache, value_cache, head_mapping, block_tables, context_lens, block_size, alibi_slopes)
     rc = lib().pb_single_query_cached_kv_attention(
         out.data_ptr(), query.data_ptr(), key_cache.data_ptr(), value_cache.data_ptr(),
         None if head_mapping is None else head_mapping.data_ptr(), float(scale), bt.data_ptr(),
@@ -59,7 +59,7 @@ def single_query_cached_kv_prev_attention(out, query, key_cache, value_cache, he
                                           context_lens, qk_maxs, exp_sums, block_size, max_context_len,
                                           alibi_slopes: Optional[torch.Tensor] = None) -> None:
     """csrc/attention.cpp:19-32: also writes the base-2 row maxima and exponent sums."""
-    bt, tail = _prepare(out, query, key_cache, value_cache, head_mapping, block_tables, context_lens, block_size, alibi_slopes)
+    (bt, ws), tail = _prepare(out, query, key_cache, value_cache, head_mapping, block_tables, context_lens, block_size, alibi_slopes)
     rc = lib().pb_single_query_cached_kv_prev_attention(
         out.data_ptr(), query.data_ptr(), key_cache.data_ptr(), value_cache.data_ptr(),
         None if head_mapping is None else head_mapping.data_ptr(), float(scale), bt.data_ptr(),
@@ -71,7 +71,7 @@ def single_query_cached_kv_post_attention(out, query, key_cache, value_cache, he
                                           context_lens, prev_qk_maxs, prev_exp_sums, block_size, max_context_len,
                                           alibi_slopes: Optional[torch.Tensor] = None) -> None:
     """csrc/attention.cpp:34-47: merges in place with the partial result already in ``out``."""
-    bt, tail = _prepare(out, query, key_cache, value_cache, head_mapping, block_tables, context_lens, block_size, alibi_slopes)
+    (bt, ws), tail = _prepare(out, query, key_cache, value_cache, head_mapping, block_tables, context_lens, block_size, alibi_slopes)
     rc = lib().pb_single_query_cached_kv_post_attention(
         out.data_ptr(), query.data_ptr(), key_cache.data_ptr(), value_cache.data_ptr(),
         None if head_mapping is None else head_mapping.data_ptr(), float(scale), bt.data_ptr(),

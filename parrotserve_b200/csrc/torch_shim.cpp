@@ -11,7 +11,7 @@
 // at the edge: void functions that write in place, launch on the current CUDA stream and raise a
 // Python RuntimeError through TORCH_CHECK on anything unsupported
 // (csrc/attention/attention_post_kernels.cu:448,500,525). The one thing the reference's kernels do
-// not need and ours do is scratch memory: the shim keeps one grow-only torch buffer per device.
+// not need and ours do is scratch memory: the shim takes it from torch's caching allocator in every call.
 //
 // Built as ONE shared object with two submodules; the package's torch_ops.py loads it and can
 // install the submodules under the reference's import names.
@@ -22,7 +22,6 @@
 #include <cstdarg>
 #include <cstdio>
 #include <map>
-#include <mutex>
 #include <string>
 #include <vector>
 
@@ -56,15 +55,11 @@ void check_rc(int rc, const char* what) {
   TORCH_CHECK(false, text("%s: invalid argument (pb_status %d)", what, rc));
 }
 
-// grow-only scratch per device (the C ABI never allocates)
-torch::Tensor& workspace(const torch::Tensor& like, size_t bytes) {
-  static std::mutex mu;
-  static std::map<int, torch::Tensor> bufs;
-  std::lock_guard<std::mutex> lock(mu);
-  torch::Tensor& b = bufs[like.get_device()];
-  if (!b.defined() || (size_t)b.numel() < bytes)
-    b = torch::empty({(int64_t)std::max<size_t>(bytes, 1 << 20)}, like.options().dtype(torch::kUInt8));
-  return b;
+// Scratch of one call (the C ABI never allocates), from the caching allocator on the current stream: freed
+// at the end of the call and handed out again behind its kernels. One buffer per device would be shared by
+// calls on different streams and of different threads.
+torch::Tensor workspace(const torch::Tensor& like, size_t bytes) {
+  return torch::empty({(int64_t)bytes}, like.options().dtype(torch::kUInt8));
 }
 
 struct Geometry {
@@ -113,7 +108,7 @@ void run_stats(StatsFn fn, const char* name, torch::Tensor& out, torch::Tensor& 
               "qk_maxs and exp_sums must be contiguous float32 tensors");
   const size_t need = pb_single_query_workspace_bytes(g.num_seqs, g.num_heads, g.head_size, block_size, g.max_blocks);
   TORCH_CHECK(need > 0, text("%s: unsupported head size %d or block size %d", name, g.head_size, block_size));
-  torch::Tensor& ws = workspace(query, need);
+  const torch::Tensor ws = workspace(query, need);
   const cudaStream_t stream = at::cuda::getCurrentCUDAStream();
   check_rc(fn(out.data_ptr(), query.data_ptr(), key_cache.data_ptr(), value_cache.data_ptr(), head_mapping.data_ptr<int32_t>(),
               scale, block_tables.data_ptr<int32_t>(), context_lens.data_ptr<int32_t>(), qk_maxs.data_ptr<float>(),
@@ -136,7 +131,7 @@ void single_query_cached_kv_attention(torch::Tensor& out, torch::Tensor& query, 
   const Geometry g = geometry(out, query, key_cache, value_cache, head_mapping, block_tables, context_lens, block_size, alibi_slopes);
   const size_t need = pb_single_query_workspace_bytes(g.num_seqs, g.num_heads, g.head_size, block_size, g.max_blocks);
   TORCH_CHECK(need > 0, text("single_query_cached_kv_attention: unsupported head size %d or block size %d", g.head_size, block_size));
-  torch::Tensor& ws = workspace(query, need);
+  const torch::Tensor ws = workspace(query, need);
   const cudaStream_t stream = at::cuda::getCurrentCUDAStream();
   check_rc(pb_single_query_cached_kv_attention(
                out.data_ptr(), query.data_ptr(), key_cache.data_ptr(), value_cache.data_ptr(), head_mapping.data_ptr<int32_t>(),

@@ -14,6 +14,7 @@ Function-level boundary (reference file:line each one replaces):
 from __future__ import annotations
 
 import ctypes as C
+import threading
 from typing import Dict, Optional, Tuple
 
 import torch
@@ -47,24 +48,44 @@ def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
 
 
 def _as_i32(t: torch.Tensor) -> torch.Tensor:
-    if t.dtype != torch.int32:
-        t = t.to(torch.int32)
-    return t.contiguous()
+    if t.dtype == torch.int32 and t.is_contiguous():
+        return t
+    return t.to(torch.int32).contiguous()
 
 
 class Workspace:
-    """Grow-only scratch buffer per device; the C ABI never allocates."""
+    """Scratch of one-shot calls (the C ABI never allocates). A buffer belongs to one thread and one stream, so that
+    the kernels of a call meet nobody else's lists and partials in it; those of the next call of that thread on that stream
+    come behind them. A thread keeps the buffers of its last few streams and gives the oldest back to torch's
+    allocator, all of them when it ends. Larger requests, and calls that are being captured (a graph
+    needs memory of its own), get a block of the allocator for themselves."""
 
-    _bufs: Dict[Tuple[str, int], torch.Tensor] = {}
+    KEEP_STREAMS = 4
+    KEEP_BYTES = 64 << 20
+
+    class _Kept(threading.local):
+        def __init__(self):
+            self.buffers = {}  # (device index, stream) -> buffer, oldest first
+
+    _kept = _Kept()
 
     @classmethod
     def get(cls, device: torch.device, nbytes: int, tag: str = "attn") -> torch.Tensor:
-        key = (tag, device.index if device.index is not None else torch.cuda.current_device())
-        buf = cls._bufs.get(key)
-        if buf is None or buf.numel() < nbytes:
-            buf = torch.empty(max(nbytes, 1 << 20), dtype=torch.uint8, device=device)
-            cls._bufs[key] = buf
-        return buf
+        index = device.index
+        if index is None:
+            index = torch.cuda.current_device()
+        if nbytes <= cls.KEEP_BYTES and not torch._C._cuda_isCurrentStreamCapturing():
+            kept = cls._kept.buffers
+            key = (index, torch._C._cuda_getCurrentRawStream(index))
+            buf = kept.get(key)
+            if buf is not None and buf.numel() >= nbytes:
+                return buf
+            kept.pop(key, None)
+            while len(kept) >= cls.KEEP_STREAMS:
+                kept.pop(next(iter(kept)))
+            buf = kept[key] = torch.empty(max(nbytes, 1 << 20), dtype=torch.uint8, device=device)
+            return buf
+        return torch.empty(nbytes, dtype=torch.uint8, device=device)
 
 
 def _kv_geometry(key_cache: torch.Tensor, value_cache: torch.Tensor):
@@ -137,18 +158,16 @@ class AttentionCall:
         p.head_size = head_size
         p.block_size = block_size
         self._keep = []
-        if suffix_tables is not None and suffix_tables.numel() > 0 and suffix_tables.shape[-1] > 0:
+        if suffix_tables is not None and suffix_tables.numel() > 0:
             suffix_tables = _as_i32(suffix_tables)
             suffix_lens = _as_i32(suffix_lens)
             _require_cuda(suffix_tables, suffix_lens)
-            if suffix_tables.dim() != 2 or suffix_tables.shape[0] != num_rows or suffix_lens.numel() != num_rows:
+            if suffix_tables.dim() != 2 or suffix_tables.size(0) != num_rows or suffix_lens.numel() != num_rows:
                 raise RuntimeError("suffix tables/lens must be [num_rows, max_blocks] / [num_rows]")
             p.suffix_lens = suffix_lens.data_ptr()
             p.suffix_tables = suffix_tables.data_ptr()
-            p.suffix_table_stride = suffix_tables.shape[1]
+            p.suffix_table_stride = suffix_tables.size(1)
             self._keep += [suffix_tables, suffix_lens]
-        else:
-            p.suffix_table_stride = 0
         if group_prefix_lens is not None and group_prefix_lens.numel() > 0:
             group_prefix_lens = _as_i32(group_prefix_lens)
             group_row_offsets = _as_i32(group_row_offsets)
@@ -158,17 +177,18 @@ class AttentionCall:
             p.num_groups = g
             p.group_row_offsets = group_row_offsets.data_ptr()
             p.group_prefix_lens = group_prefix_lens.data_ptr()
+            _require_cuda(group_prefix_lens, group_row_offsets)
             self._keep += [group_prefix_lens, group_row_offsets]
             if group_tables is not None and group_tables.numel() > 0:
                 group_tables = _as_i32(group_tables)
                 if group_tables.dim() == 1:
                     group_tables = group_tables.unsqueeze(0)
-                if group_tables.shape[0] != g:
+                if group_tables.size(0) != g:
                     raise RuntimeError("group_tables must be [num_groups, max_prefix_blocks]")
                 p.group_tables = group_tables.data_ptr()
-                p.group_table_stride = group_tables.shape[1]
+                p.group_table_stride = group_tables.size(1)
+                _require_cuda(group_tables)
                 self._keep.append(group_tables)
-            _require_cuda(*self._keep)
         if seg_kv_lens is not None and seg_kv_lens.numel() > 0:
             # causal segments: the new tokens of prefill requests (see pb_attn_params in the header)
             seg_kv_lens, seg_row_offsets, seg_tables = _as_i32(seg_kv_lens), _as_i32(seg_row_offsets), _as_i32(seg_tables)
@@ -214,31 +234,32 @@ class AttentionCall:
             p.slot_is_i64 = 1 if slot_mapping.dtype == torch.int64 else 0
             self._keep.append(slot_mapping)
         self._has_slots = slot_mapping is not None
-        p.dense_min_rows = dense_min_rows
-        p.suffix_chunk_blocks = suffix_chunk_blocks
-        p.prefix_chunk_blocks = prefix_chunk_blocks
-        p.dense_ctas = dense_ctas
-        p.dense_row_tile = dense_row_tile
+        if dense_min_rows or suffix_chunk_blocks or prefix_chunk_blocks or dense_ctas or dense_row_tile:
+            p.dense_min_rows = dense_min_rows
+            p.suffix_chunk_blocks = suffix_chunk_blocks
+            p.prefix_chunk_blocks = prefix_chunk_blocks
+            p.dense_ctas = dense_ctas
+            p.dense_row_tile = dense_row_tile
         self.params = p
-        nbytes = lib().pb_attn_workspace_bytes(C.byref(p))
+        self._params_ref = C.byref(p)
+        nbytes = lib().pb_attn_workspace_bytes(self._params_ref)
         if nbytes == 0:
             raise _lib.PbError(_lib.PB_ERR_UNSUPPORTED, "pb_attn_workspace_bytes",
                                f"head_size={head_size} block_size={block_size} dtype={dtype}")
         self.workspace_bytes = nbytes
         # A planned call keeps its work lists in the workspace between plan() and every run(), so it owns
-        # its buffer; only the one-shot wrappers (plan + run in one library call) share the per-device one.
+        # its buffer; only the one-shot wrappers (plan + run in one library call) share a kept one.
         if workspace is not None:
             self.workspace = workspace
         elif shared_workspace:
             self.workspace = Workspace.get(device, nbytes)
         else:
             self.workspace = torch.empty(nbytes, dtype=torch.uint8, device=device)
-        if self.workspace.numel() < nbytes:
+        p.workspace_bytes = have = self.workspace.numel()
+        if have < nbytes:
             raise _lib.PbError(_lib.PB_ERR_WORKSPACE, "AttentionCall")
         p.workspace = self.workspace.data_ptr()
-        p.workspace_bytes = self.workspace.numel()
         self._planned = False
-        self._params_ref = C.byref(p)
         self._q_shape = (num_rows, num_heads, head_size)
 
     def _bind(self, query, out, key_cache, value_cache, qk_max=None, exp_sum=None, stats_mode=_lib.PB_STATS_NONE):
@@ -517,6 +538,7 @@ def _single_group_meta(device: torch.device, prefix_len: int, num_rows: int):
     hit = _const_cache.get(key)
     if hit is None:
         if len(_const_cache) > 256:
+            torch.cuda.synchronize(device)  # calls on other streams may still read what is given back here
             _const_cache.clear()
         hit = (
             torch.tensor([0, num_rows], dtype=torch.int32, device=device),

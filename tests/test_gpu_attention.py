@@ -887,3 +887,93 @@ def test_default_row_tile(new, decode, groups, tile):
     """Row-tile pairs are the default for batches of long prefills in large groups only (dense items of the plan)."""
     items = {t: _planned_header(new, decode, groups, dense_row_tile=t)[2] for t in (0, 128, 256)}
     assert items[128] != items[256] and items[0] == items[tile]
+
+
+@pytest.mark.parametrize("entry", ["wrappers", "compiled", "threads"])
+def test_one_shot_calls_side_by_side(entry):
+    """Different one-shot calls at the same time, on two streams or from two threads on one, each many times: every
+    result is the one of the call on its own. (Scratch that they share would mix their lists and partials.)"""
+    import threading
+
+    from parrotserve_b200 import torch_ops
+
+    problems = [_mini(torch.float16, 8, 300, [200 + 7 * i for i in range(24)], nb=560, seed=70),
+                _mini(torch.float16, 4, 0, [1 + 90 * i for i in range(16)], nb=720, seed=71)]
+    i32 = lambda a: torch.tensor(a, dtype=torch.int32, device=DEV)
+
+    def prepared(q, kc, vc, meta):
+        plens, gt, offs, sl, st = (i32(meta[n]) for n in ("plens", "gt", "offs", "sl", "st"))
+        hm = torch.arange(q.shape[1], dtype=torch.int32, device=DEV)
+        if entry != "compiled":
+            return lambda: pb.flash_paged_attention_grouped(q, kc, vc, None, plens, gt, offs, sl, st)
+        ops, _ = torch_ops.load()
+
+        def call():
+            out = torch.empty_like(q)
+            ops.single_query_cached_kv_attention(out, q, kc, vc, hm, 128 ** -0.5, st, st, sl, sl, 16, st.shape[1] * 16, None)
+            return out
+        return call
+
+    calls = [prepared(*p) for p in problems]
+    alone = [c() for c in calls]
+    torch.cuda.synchronize()
+    outs = [[], []]
+    if entry == "threads":
+        start = threading.Barrier(2)
+
+        def work(k):
+            start.wait()
+            for _ in range(60):
+                outs[k].append(calls[k]())
+
+        threads = [threading.Thread(target=work, args=(k,)) for k in (0, 1)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+    else:
+        streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+        for _ in range(40):
+            for k in (0, 1):
+                with torch.cuda.stream(streams[k]):
+                    outs[k].append(calls[k]())
+    torch.cuda.synchronize()
+    for k in (0, 1):
+        assert len(outs[k]) >= 40
+        for out in outs[k]:
+            assert torch.equal(out, alone[k])
+
+
+def test_kept_scratch_is_bounded_and_not_captured():
+    """The scratch a thread keeps for one-shot calls: one buffer per stream for the last few streams, none for
+    large calls, and none of it in a captured graph, which still replays after the buffers were replaced."""
+    from parrotserve_b200.ops import Workspace
+
+    dev = torch.device(DEV)
+    streams = [torch.cuda.Stream() for _ in range(Workspace.KEEP_STREAMS + 3)]
+    for s in streams:
+        with torch.cuda.stream(s):
+            ws = Workspace.get(dev, 1000)
+            assert Workspace.get(dev, 2000).data_ptr() == ws.data_ptr()
+            assert Workspace.get(dev, Workspace.KEEP_BYTES + 1).data_ptr() != ws.data_ptr()
+    assert len(Workspace._kept.buffers) <= Workspace.KEEP_STREAMS
+    q, kc, vc, meta = _mini(torch.float16, 4, 100, [30, 5, 64, 17], nb=64, seed=72)
+    i32 = lambda a: torch.tensor(a, dtype=torch.int32, device=DEV)
+    plens, gt, offs, sl, st = (i32(meta[n]) for n in ("plens", "gt", "offs", "sl", "st"))
+    call = lambda: pb.flash_paged_attention_grouped(q, kc, vc, None, plens, gt, offs, sl, st)
+    want = call()
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        call()
+        side.synchronize()
+        kept = Workspace.get(dev, 1000).data_ptr()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=side):
+            out = call()
+        assert Workspace.get(dev, 1000).data_ptr() == kept
+        Workspace._kept.buffers.clear()
+        filler = [torch.full((1 << 20,), 0x7F, dtype=torch.uint8, device=DEV) for _ in range(4)]
+        out.zero_()
+        graph.replay()
+        side.synchronize()
+    assert torch.equal(out, want) and len(filler) == 4
