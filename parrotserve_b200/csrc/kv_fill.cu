@@ -452,6 +452,11 @@ __global__ void __launch_bounds__(128) fill_window_kernel(
     }
   };
 
+  // lane l: the slot of token first - 1 + l (negative: none, or outside the cache); asked for before q is worked on
+  const long long my = first - 1 + lane;
+  long long slot = (kcache != nullptr && my >= 0 && my < T_tok) ? load_slot(slots, is64, my) : -1;
+  if (slot >= num_blocks * B) slot = -1;
+
   if (do_q) {  // q in place; with no cache k too (eight lanes: 128 contiguous bytes of a row)
     const long long tok = first + warp * 4 + (lane >> 3);
     if (tok < T_tok) {
@@ -475,11 +480,6 @@ __global__ void __launch_bounds__(128) fill_window_kernel(
     }
   }
   if (h0 >= H || kcache == nullptr || !(do_k || do_v)) return;
-
-  // lane l: the slot of token first - 1 + l (negative: none, or outside the cache)
-  const long long my = first - 1 + lane;
-  long long slot = (my >= 0 && my < T_tok) ? load_slot(slots, is64, my) : -1;
-  if (slot >= num_blocks * B) slot = -1;
 
   // ---- K: token `i` of the window, chunks g, g + 8, ... ----
   const int i = (lane & 7) + 8 * (warp & 1), g = (lane >> 3) + 4 * (warp >> 1);
