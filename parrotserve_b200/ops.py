@@ -565,7 +565,7 @@ def flash_paged_attention_grouped(
     (a single LCA per batch, parrot/engine/builtin/attn_func.py:441-459)."""
     num_rows, num_heads, head_size = query.shape
     if out is None:
-        out = torch.empty((num_rows, num_heads, head_size), dtype=query.dtype, device=query.device)
+        out = query.new_empty((num_rows, num_heads, head_size))
     if num_rows == 0:
         return out
     call = AttentionCall(
@@ -614,7 +614,7 @@ def vllm_paged_attention(
 ) -> torch.Tensor:
     """Unshared paged decode attention (parrot/engine/builtin/kernels/vllm/paged_attention.py:12-38)."""
     num_rows, num_heads, head_size = query.shape
-    out = torch.empty((num_rows, num_heads, head_size), dtype=query.dtype, device=query.device)
+    out = query.new_empty((num_rows, num_heads, head_size))
     if num_rows == 0:
         return out
     call = AttentionCall(
