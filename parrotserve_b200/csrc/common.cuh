@@ -77,8 +77,9 @@ struct DnItem {       // one tile of query rows and the kv tokens they attend in
   // request's own context (seg_tables + tbl2_off, nblk/ntok/causal_base above). nt1 == 0: one piece,
   // in group_tables (causal_base == 0) or seg_tables (causal_base > 0) at tbl_off.
   int32_t nt1, nblk1, ntok1, tbl2_off;
-  int32_t flags;  // kDnDirect: none of the item's rows has any other partial (no suffix, no other item), so a CTA that holds ALL kv tiles of (item, head) writes the finished,
-                  // normalised output rows itself and the merge skips them
+  int32_t flags;  // kDnDirect: none of the item's rows has any other partial (no suffix, no other item), so a CTA
+                  // that holds ALL kv tiles of (item, head) writes the finished, normalised output rows itself
+                  // and the merge skips them
   int32_t fixed;  // positions of the tile order in front of every head's tiles (kCausalFixedTiles or 0)
   int32_t pad[2];
 };
@@ -88,8 +89,8 @@ constexpr int32_t kDnDirect = 1;
 // pipeline, the epilogue. Causal items have from one kv tile to dozens, so CTAs with equal shares of the
 // tiles alone had very unequal work (those with the short row tiles of a prefill up to ten times as many
 // epilogues, and the SMs were busy 54 % of the kernel's time). Four prompts of 1500..3000 tokens, single row
-// tiles: 645 us with 0, 483 with 2, 485 with 3, 488 with 5; row-tile pairs: 426 with 2, 417 with 3, 422 with 4; 16
-// prefills under a shared prefix are indifferent (1135, 1134, 1132).
+// tiles: 645 us with 0, 483 with 2, 485 with 3, 488 with 5; row-tile pairs: 426 with 2, 417 with 3, 422 with 4;
+// prefills under a shared prefix are indifferent.
 // Items without a causal mask are equally long within a group; their tiles are split as they are.
 constexpr int32_t kCausalFixedTiles = 3;
 constexpr int32_t kDnOuter = 2;   // the item walks an outer prefix group (outer_tables, outer partial range)

@@ -98,7 +98,7 @@ __device__ __forceinline__ void exp_pack32(const uint32_t* v, int nvalid, float 
 #pragma unroll
   for (int i = 0; i < 32; i += 2) {
     float e0 = __uint_as_float(v[i]), e1 = __uint_as_float(v[i + 1]);
-    fma_pair(e0, e1, scale, -m);  // (a packed instruction: four prompts of 1500..3000 tokens 440 -> 432 us)
+    fma_pair(e0, e1, scale, -m);
     e0 = fast_exp2(e0);
     e1 = fast_exp2(e1);
     if (kMasked) {
@@ -255,7 +255,8 @@ dense_pair_kernel(const AttnDev d, const __grid_constant__ CUtensorMap vmap, con
     // the second of the two commits on it. On pair items they issue in turns (0, 1, 0, 1, ...): issued
     // together, the MMAs of both tiles share the pipe and end together, and the two softmax groups fall into
     // step, both at the exponentials, then both waiting. 16 prefills of 256..1024 tokens with 240 decodes under a
-    // 2048-token prefix: 1203 -> 1132 us; four prompts of 1500..3000 tokens unchanged (415, with 3 fixed tiles).
+    // 2048-token prefix: 6 % less (1203 -> 1132 us on one GPU; others of its kind take up to 1220 now); four prompts of
+    // 1500..3000 tokens unchanged (415, with 3 fixed tiles).
     // The operand descriptors are built once; an MMA adds its offset to the address field. (Built per
     // MMA, the descriptor arithmetic of the issuing thread costs more than the MMA itself.)
     //   Q_x: [64-element half][row][128 B], 128-byte swizzle -> SBO 1024 (8-row groups)

@@ -214,8 +214,8 @@ __global__ void __launch_bounds__(kPlanThreads, 1) plan_kernel(const AttnDev d, 
   __shared__ unsigned long long sq_blocks;  // blocks all single-query items stream, per head
   // The kernel before this one may still be at work, and it may own the very memory this call's workspace lies
   // in: a merge of another call on the same scratch, whose partials are where this call's lists go, or the
-  // stores of an output whose memory has been handed out again. Until pdl_wait() only lengths and offsets are read and nothing
-  // is written outside shared memory; faults found while counting are kept here.
+  // stores of an output whose memory has been handed out again. Until pdl_wait() only lengths and offsets are
+  // read and nothing is written outside shared memory; faults found while counting are kept here.
   __shared__ int32_t count_hdr[kHdrStatus + 1];
   AttnDev c = d;
   c.hdr = count_hdr;
@@ -316,7 +316,11 @@ __global__ void __launch_bounds__(kPlanThreads, 1) plan_kernel(const AttnDev d, 
     // the streaming kernel). A dense tile is weighted: giving the dense kernel too many SMs costs
     // little, because its CTAs retire early and the single-query kernel takes their SMs over, while
     // too few make it the long pole.
-    const double td = kDenseTileWeight * (double)total_tiles * d.num_heads * (RT / 128);  // a pair item's kv tile is two tiles of work
+    // (In positions of the tile order, the fixed ones included, twice as many where items are row-tile pairs: what an
+    // (item, head) costs beside its tiles keeps an SM busy too, and a lone row tile costs nearly what a pair does. With
+    // the kv tiles of row tiles of 128 rows alone: 64 groups x 16 decode rows and a 512-token prefill 461 us against 417,
+    // 4 groups x 250 and a 2000-token one 421 against 382.)
+    const double td = kDenseTileWeight * (double)total_tiles * d.num_heads * (RT / 128);
     const double ts = (double)sq_blocks * d.num_heads / kDenseTileBlocks;
     const int sms = d.num_sms;
     int c = sms;
